@@ -755,9 +755,9 @@ def run_ours(args, wl):
                            **executed_fp32(ph, shape, patch, stride, main["ranks"], fp32_peak, args.form)),
             cpu_baseline=cpu,
             clocks=main["clocks"],
-            gpu_launches=6 * args.steps,
+            gpu_launches=5 * args.steps,
             gpu_launches_note="per step: center, gram (column TMA or tensor), eigh, eigh_refine, "
-                              "refine_advance, recon (plus two status memsets)",
+                              "recon (plus two status memsets)",
             wall_s_timed_region=main["wall"],
         )
         if "accuracy" in main:
@@ -889,9 +889,9 @@ def run_sharded(args, wl):
     flush = torch.empty(256 << 20, dtype=torch.uint8, device=dev)
     stream = torch.cuda.current_stream(dev)
     P_total = n_patches(gshape, patch, stride)
-    # this rank's kernels per step: centre, Gram, eigensolve, refine, refine cursor, and one
+    # this rank's kernels per step: centre, Gram, eigensolve, refine, and one
     # reconstruction per non-empty part (halo out, interior, halo in)
-    launches = 5 + int(slab.halo_out.numel() > 0) + int(slab.own[1] - slab.own[0] > slab.plan.hin) + \
+    launches = 4 + int(slab.halo_out.numel() > 0) + int(slab.own[1] - slab.own[0] > slab.plan.hin) + \
         int(slab.plan.hin > 0)
 
     def step():
@@ -1048,7 +1048,7 @@ def run_batched(args):
         steps=args.steps, warmup=args.warmup, ms_per_step=ms, higher_is_better=True, dtype="f32", data="synthetic",
         single_volume_ms_sum=sum(single), vs_single_volumes=sum(single) / ms,
         gpu_launches=launches * args.steps, launches_per_batch=launches,
-        launches_one_by_one=6 * len(shapes),
+        launches_one_by_one=5 * len(shapes),
         config=dict(volumes=args.volumes, seed=args.seed, patches=P, algorithmic_tflop=flops / 1e12,
                     shapes=[[list(r["shape"]), r["patch"][0], r["stride"]] for r in shapes],
                     note="one lrd_batch_denoise CUDA-graph launch per step: packed kernels, one grid per phase and "

@@ -18,6 +18,7 @@
 #include "center.cuh"
 #include "eigh.cuh"
 #include "eigh_cta.cuh"
+#include "eigh_refine.cuh"
 #include "eigh_reg.cuh"
 #include "gram_z.cuh"
 #include "lrd_common.cuh"
@@ -37,7 +38,7 @@ struct alignas(64) BatchVol {
   float* wgt;
   float* sig2;
   int* status;
-  int* refine;           // [count, refined, 62 unused, ids...]
+  int* refine;           // [count, 63 unused, ids...]
   Geom g;
   AxisTables tab;
   int ring;              // gram_z window slots
@@ -57,13 +58,12 @@ __device__ __forceinline__ int batch_find(const long long* __restrict__ off, int
   return lo;
 }
 
-// Clears every volume's status word and near-tie queue cursor (what the
+// Clears every volume's status word and near-tie queue count (what the
 // single-volume call does with two memsets).
 __global__ void batch_reset_kernel(const BatchVol* __restrict__ vols, int n) {
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
     *vols[i].status = 0;
     vols[i].refine[0] = 0;
-    vols[i].refine[1] = 0;
   }
 }
 
@@ -109,17 +109,13 @@ __global__ void __launch_bounds__(TMAX) eigh_cta_batch_kernel(const BatchVol* __
 }
 
 // Float64 near-tie pass: each listed volume's queue is worked by its blocks.
-__global__ void eigh_refine_batch_kernel(const BatchVol* __restrict__ vols, const int* __restrict__ list,
-                                         const long long* __restrict__ off, int n) {
+__global__ void __launch_bounds__(kRefineThreads)
+    eigh_refine_batch_kernel(const BatchVol* __restrict__ vols, const int* __restrict__ list,
+                             const long long* __restrict__ off, int n) {
   const int i = batch_find(off, n, blockIdx.x);
   const BatchVol& V = vols[list[i]];
   eigh_refine_body(V.vol, V.xc, V.gv, nullptr, V.rank, V.wgt, V.sig2, V.g, V.tab, V.refine, V.refine + 64,
                    (int)(blockIdx.x - off[i]), (int)(off[i + 1] - off[i]));
-}
-
-__global__ void refine_advance_batch_kernel(const BatchVol* __restrict__ vols, int n) {
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
-    vols[i].refine[1] = vols[i].refine[0];
 }
 
 template <int Q, bool ACCURATE>

@@ -2,7 +2,7 @@
 //
 // One warp per matrix: Householder tridiagonalisation, bisection on Sturm
 // counts, MP rank (mp_rank, eigh.cuh), inverse iteration, back-transform,
-// Gram-Schmidt (the steps of eigh_mp_block, eigh.cuh), with the data placed
+// Gram-Schmidt (the float64 pass of eigh_refine.cuh takes the same steps), with the data placed
 // for a warp:
 //
 //  * lane l holds rows l and l + 32 of the working matrix in registers

@@ -16,6 +16,7 @@
 #include "../../include/lrd.h"
 #include "center.cuh"
 #include "eigh.cuh"
+#include "eigh_refine.cuh"
 #include "eigh_reg.cuh"
 #include "eigh_cta.cuh"
 #include "noise.cuh"
@@ -470,7 +471,7 @@ int run_gram(const lrd_plan* P, char* ws, float* d_gram, cudaStream_t st, long l
 
 // Float32 eigensolver over patches [p_lo, p_hi) (-1 = all), then the float64
 // pass over the near-tie patches it queued (the queue lives in the workspace:
-// [count, refined, 62 unused, ids...]; the centred volume there is the one
+// [count, 63 unused, ids...]; the centred volume there is the one
 // the Gram was formed from). ``reset`` clears the queue first.
 int run_eigh(const lrd_plan* P, char* ws, const float* d_gram, float* d_vecs, float* d_lam, int32_t* d_rank,
              float* d_wgt, cudaStream_t st, long long p_lo = 0, long long p_hi = -1, bool reset = true,
@@ -512,13 +513,9 @@ int run_eigh(const lrd_plan* P, char* ws, const float* d_gram, float* d_vecs, fl
     if (rc) return rc;
   }
   const float* xc = reinterpret_cast<const float*>(ws + P->off_xc);
-  lrd::eigh_refine_kernel<<<P->refine_blocks, 128, P->smem_refine, st>>>(d_vol, xc, d_vecs, d_lam, d_rank, d_wgt,
-                                                                        sig2,
-                                                                        P->g, P->tab, rcount, rids);
-  int rc = launch_check("eigh_refine_kernel launch");
-  if (rc) return rc;
-  lrd::refine_advance_kernel<<<1, 1, 0, st>>>(rcount);
-  return launch_check("refine_advance_kernel launch");
+  lrd::eigh_refine_kernel<<<P->refine_blocks, lrd::kRefineThreads, P->smem_refine, st>>>(
+      d_vol, xc, d_vecs, d_lam, d_rank, d_wgt, sig2, P->g, P->tab, rcount, rids);
+  return launch_check("eigh_refine_kernel launch");
 }
 
 // Reconstruction of bricks [b_lo, b_hi) (x-major brick index; -1 = all).
@@ -807,12 +804,12 @@ int create_plan(const lrd_problem* pr, const std::vector<int32_t>* x_corners, lr
   if (!rc) rc = set_smem((const void*)lrd::gram_kernel, P->smem_gram);
   if (!rc && P->use_gramz) rc = set_smem(gramz_kernel_ptr(P->gramz_ks), P->smem_gramz);
   if (!rc && P->use_gramtc) rc = set_smem(gramtc_kernel_ptr(P->gramtc_bf16), P->smem_gramtc);
-  P->smem_refine = lrd::eigh_refine_smem_bytes(T, pr->pz);
+  P->smem_refine = lrd::eigh_refine_smem_bytes(T);
   if (!rc) rc = set_smem((const void*)lrd::eigh_refine_kernel, P->smem_refine);
   {
     int sms = 148;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    P->refine_blocks = std::max(1, std::min<int>(2 * sms, (int)std::min<long long>(g.npatch, 1 << 20)));
+    P->refine_blocks = std::max(1, std::min<int>(sms, (int)std::min<long long>(g.npatch, 1 << 20)));
     P->sms = sms;
     int per_sm = 0;
     if (!rc && P->use_gramz) {
