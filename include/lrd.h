@@ -85,8 +85,8 @@ enum lrd_form {
  * voxel (recon_split: 1, 2 or 4); 0 = chosen by the plan's cost model (the
  * autotuner fills them in). These change speed only: every voxel's arithmetic
  * and accumulation order are the same for any brick and split.
- * ``gram_split``: threads sharing a 4x4 block of the column Gram (1, 2 or 4,
- * each summing every n-th voxel row); ``eigh_block``: 1 = one warp per
+ * ``gram_split`` n: 2n threads share an 8x8 block of the column Gram (n = 1, 2
+ * or 4, each thread summing every 2n-th voxel row); ``eigh_block``: 1 = one warp per
  * matrix (T <= 64), 2 = one CTA of 64 / 96 / 128 threads per matrix; 0 = the
  * plan's choice for both. These two change the float32 rounding of the Gram
  * and the eigenvalues (ranks stay the same: near-ties are decided in FP64

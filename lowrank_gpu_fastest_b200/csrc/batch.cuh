@@ -42,6 +42,7 @@ struct alignas(64) BatchVol {
   Geom g;
   AxisTables tab;
   int ring;              // gram_z window slots
+  int cut;               // window ranges a column is cut into (1: whole columns)
 };
 
 // Index i of the list entry whose block range holds block b (off has n + 1
@@ -75,17 +76,18 @@ __global__ void center_batch_kernel(const BatchVol* __restrict__ vols, const int
   center_body(V.vol, V.xc, V.mean, nvox, V.g.nt, (long long)blockIdx.x - off[i]);
 }
 
-// Column Gram, every column of each listed volume (no short-last-wave cut:
-// the batch's columns fill the device).
+// Column Gram, every column of each listed volume (no short-last-wave cut: the
+// batch's columns fill the device; only a ring that does not fit is cut).
 template <int KS>
-__global__ void __maxnreg__(64) gram_z_batch_kernel(const BatchVol* __restrict__ vols, const int* __restrict__ list,
+__global__ void __launch_bounds__(kGramzMaxThreads) gram_z_batch_kernel(const BatchVol* __restrict__ vols, const int* __restrict__ list,
                                                     const long long* __restrict__ off, int n) {
   const int i = batch_find(off, n, blockIdx.x);
   const BatchVol& V = vols[list[i]];
   if (threadIdx.x == 0)  // the map was written by a copy before this launch; order it for the TMA unit
     asm volatile("fence.proxy.tensormap::generic.acquire.gpu [%0], 128;\n" ::"l"(&V.map) : "memory");
   const long long ncols = (long long)V.g.ncx * V.g.ncy;
-  gram_z_body<KS>(&V.map, V.gv, V.g, V.tab, 0, V.ring, (int)ncols, 1, V.status, (int)(blockIdx.x - off[i]));
+  gram_z_body<KS>(&V.map, V.gv, V.g, V.tab, 0, V.ring, V.cut > 1 ? 0 : (int)ncols, V.cut, V.status,
+                  (int)(blockIdx.x - off[i]));
 }
 
 template <int TMAX>

@@ -7,20 +7,33 @@
 // contain z; this kernel computes each H(z) once and adds it into every active
 // window, which cuts the FFMA work by that factor (3.2x at 11^3 / stride 3).
 //
-// Layout: one CTA per (x-corner, y-corner) column; ``ks`` adjacent threads
-// (lanes of one warp) share the 4x4 block G[4bi:4bi+4, 4bj:4bj+4], bi <= bj,
-// each summing every ks-th voxel row of a plane, combined by shuffles (a
-// K-split: ks times the warps per column for latency hiding). The block size
-// is rounded up to whole warps; the extra threads only join the shuffles and
-// barriers. The column's planes are
-// streamed into a two-slot shared-memory ring by TMA (one 4D box (T, 1, py, px)
-// of the centred volume per plane, completion on an mbarrier); the window
-// accumulators of the active windows live in shared memory (a ring of
-// ``ring`` slots, slot = window index mod ring). A plane's partial Gram is
-// summed in float32 over its px*py voxels (FFMA), then added to the windows in
-// float32; a window is written out (and its slot cleared) after its last plane.
-// The K = px*py*pz sum therefore rounds as a two-level blocked sum, plane then
-// window (the per-patch kernel rounds as x-plane then float64 window).
+// Layout: one CTA per (x-corner, y-corner) column; KS lanes of a warp share an
+// 8 x 8 block of the upper block triangle, each summing every KS-th voxel row.
+// The column's planes are streamed into a two-slot shared-memory ring by TMA (one
+// 4D box (T, 1, py, px) of the centred volume per plane, completion on an
+// mbarrier); the window accumulators of the active windows live in shared memory
+// (a ring of ``ring`` slots, slot = window index mod ring).
+//
+// A 4 x 4 block reads 2 bytes of shared memory per FMA, and LDS.128 returns 128
+// bytes a clock to an SM's 128 FMA lanes: that bound the kernel (77% of the shared
+// data pipe, 38% of the FMA pipe). An 8 x 8 block reads 1 byte per FMA. The packed
+// FMA (two IEEE FMAs) halves the issue slots: 107 instead of 94 FMA a clock at 12
+// warps per SM in a loop of nothing else. What bounds it now is 9 to 12 warps per
+// SM that stop at the plane barrier and at the flush below. Gram phase on B200:
+// 96x96x48x48 / 11^3 / stride 3 0.61 -> 0.52 ms, 96x96x48x32 / 5^3 / stride 1 1.58
+// -> 1.40, 101x87x43x64 / 7^3 / stride 2 1.21 -> 0.98, 64x64x48x96 / 11^3 / stride 3
+// 0.99 -> 0.70; 128x128x64x96 / 11^3 / stride 2, whose full ring does not fit
+// shared memory and which ran a CTA per patch, 68.1 -> 10.2.
+//
+// Planes that lie in the same windows (two of three at 11^3 / stride 3) are summed
+// in registers; at the last of them the KS lanes' partial sums are combined by
+// halving exchanges and added to the windows in float32, and a window is written
+// out (and its slot cleared) after its last plane. The K = px*py*pz sum therefore
+// rounds as a blocked sum: rows of a plane group, lanes, window.
+// Tried and dropped (headline ms): a producer warp with chunks of x-rows and no
+// CTA barrier 0.59 (its warp leaves one of the SM's four schedulers idle), the
+// same with thread 0 of the first warp as producer 0.63, the next row's loads
+// moved ahead of this row's products by hand 0.81.
 //
 // Every mbarrier wait is bounded by a %globaltimer deadline. On expiry the
 // kernel records LRD_STATUS_TMA_TIMEOUT in the status word (the result is
@@ -57,7 +70,7 @@ __device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes) {
 __device__ __forceinline__ bool mbar_wait_bounded(uint32_t bar, uint32_t parity, int* status,
                                                   int code = kStatusTmaTimeout,
                                                   unsigned long long limit_ns = kWaitNs) {
-  const unsigned long long t0 = globaltimer_ns();
+  unsigned long long t0 = 0;  // the clock is read only once the first try has failed
   for (;;) {
     uint32_t ok;
     asm volatile(
@@ -66,7 +79,9 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint32_t bar, uint32_t parity,
         : "r"(bar), "r"(parity)
         : "memory");
     if (ok) return true;
-    if (globaltimer_ns() - t0 > limit_ns) {
+    if (t0 == 0) {
+      t0 = globaltimer_ns();
+    } else if (globaltimer_ns() - t0 > limit_ns) {
       atomicOr(status, code);
       return false;
     }
@@ -82,39 +97,50 @@ __device__ __forceinline__ void tma_load_4d(uint32_t dst, const CUtensorMap* map
       : "memory");
 }
 
-// After a wait gave up: wait (bounded) for the copies still in flight into the
-// CTA's shared memory - the one whose wait gave up (``a``) and the one issued
-// after it (``b``) - before the CTA exits.
-__device__ __noinline__ void drain_copies(bool wait_a, uint32_t bar_a, uint32_t par_a, bool wait_b,
-                                          uint32_t bar_b, uint32_t par_b, int* status) {
-  if (wait_a) mbar_wait_bounded(bar_a, par_a, status);
-  if (wait_b) mbar_wait_bounded(bar_b, par_b, status);
-}
-
 __host__ __device__ inline size_t gramz_plane_floats(int rows, int T) {
   return ((size_t)rows * T + 31) & ~size_t(31);  // 128-byte multiple
 }
 
-// Dynamic shared memory: two plane slots, ring * 16 * nblk float window
-// accumulators (nblk = 4x4 blocks of the upper triangle), two mbarriers.
-__host__ __device__ inline size_t gramz_smem_bytes(int rows, int T, int ring, int nblk) {
-  return sizeof(float) * (2 * gramz_plane_floats(rows, T) + (size_t)ring * 16 * nblk) + 16;
+// 8 x 8 blocks of the upper block triangle: block b of nb = ceil(T / 8) owns the
+// 4-frame quads b and b + nb (the second one absent at the end of an odd count).
+__host__ __device__ inline int gramz_nb(int T) { return ((T >> 2) + 1) >> 1; }
+__host__ __device__ inline int gramz_nblk(int T) {
+  const int nb = gramz_nb(T);
+  return nb * (nb + 1) / 2;
 }
 
-// Threads of a column CTA for T frames and K-split ks: nb*(nb+1)/2 blocks
-// (nb = T/4) times ks, rounded up to whole warps.
+// Threads of a column CTA for T frames and K-split ks: the blocks, 32 / ks to a
+// warp, times ks.
 __host__ __device__ inline int gramz_threads(int T, int ks) {
-  const int nb = T >> 2;
-  return ((nb * (nb + 1) / 2 * ks) + 31) & ~31;
+  const int per_warp = 32 / ks;
+  return 32 * ((gramz_nblk(T) + per_warp - 1) / per_warp);
+}
+
+// Dynamic shared memory: two plane slots, ``ring`` window accumulators (64 floats
+// per block), two mbarriers.
+__host__ __device__ inline size_t gramz_smem_bytes(int px, int py, int T, int ring) {
+  return sizeof(float) * (2 * gramz_plane_floats(px * py, T) + (size_t)ring * 64 * gramz_nblk(T)) + 2 * sizeof(uint64_t);
+}
+
+// (c0, c1) += (a, a) * (b0, b1): two IEEE FMAs in one instruction.
+__device__ __forceinline__ void fma2(float2& c, float2 a, float2 b) {
+  unsigned long long ra, rb, rc;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(ra) : "f"(a.x), "f"(a.y));
+  asm("mov.b64 %0, {%1, %2};" : "=l"(rb) : "f"(b.x), "f"(b.y));
+  asm("mov.b64 %0, {%1, %2};" : "=l"(rc) : "f"(c.x), "f"(c.y));
+  asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(rc) : "l"(ra), "l"(rb));
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(c.x), "=f"(c.y) : "l"(rc));
 }
 
 // grid: nfull + (columns - nfull) * nsplit CTAs; block: gramz_threads(T, KS)
-// (T % 4 == 0, KS in {1, 2, 4}). CTA b < nfull computes every window of column
+// (T % 4 == 0, KS in {2, 4, 8}). CTA b < nfull computes every window of column
 // col0 + b; the columns after the first nfull are each cut into nsplit units
-// of consecutive windows (a unit reads only the planes of its windows), so a
-// launch whose last wave would hold a few whole columns spreads that tail
-// over many SMs. A window's planes are added in the same order either way: the
-// result does not depend on the cut. ``col0`` = first column (x-major index
+// of consecutive windows (a unit reads only the planes of its windows; it needs
+// min(windows active at a plane, windows of the unit) <= ring), so a launch
+// whose last wave would hold a few whole columns spreads that tail over many
+// SMs, and a ring that does not fit shared memory is cut to one that does. The
+// planes are grouped by the column's windows, not the unit's, so the result
+// does not depend on the cut. ``col0`` = first column (x-major index
 // ci * ncy + cj); ``gram`` points at the Gram block of the launch's first
 // patch (patch index col0 * ncz).
 // Body of one CTA (index ``bid``); ``xmap`` points at the tensor map (a kernel
@@ -124,154 +150,216 @@ template <int KS>
 __device__ __forceinline__ void gram_z_body(const CUtensorMap* xmap, float* __restrict__ gram, const Geom& g,
                                             const AxisTables& tab, long long col0, int ring, int nfull, int nsplit,
                                             int* status, int bid) {
-  constexpr int ks = KS;
+  static_assert(KS == 2 || KS == 4 || KS == 8, "threads per block");
+  constexpr int BW = 32 / KS;  // blocks per warp: lane = kq * BW + block
+  constexpr int NR = 8 / KS;   // rows of its block a thread ends up with: kq * NR ...
   extern __shared__ __align__(128) float smz[];
   const int T = g.nt;
   const int rows = g.px * g.py;
   const size_t pf = gramz_plane_floats(rows, T);
-  float* plane0 = smz;
-  float* plane1 = smz + pf;
-  const int nb = T >> 2;
-  const int nblk = nb * (nb + 1) / 2;
-  float* win = smz + 2 * pf;  // [ring][16][nblk]
+  const int nq = T >> 2, nb = gramz_nb(T), nblk = gramz_nblk(T);
   const int nthreads = blockDim.x;
-  uint64_t* bars = reinterpret_cast<uint64_t*>(win + (size_t)ring * 16 * nblk);
-  const uint32_t bar0 = (uint32_t)__cvta_generic_to_shared(&bars[0]);
-  const uint32_t bar1 = (uint32_t)__cvta_generic_to_shared(&bars[1]);
+  const int nown = nblk * KS;                             // threads that own a share of a block
+  float4* win = reinterpret_cast<float4*>(smz + 2 * pf);  // [ring][2 NR][nown]
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smz + 2 * pf + (size_t)ring * 64 * nblk);
+  const uint32_t bar0 = (uint32_t)__cvta_generic_to_shared(bars);
 
   // this CTA's column and windows [wlo, whi]
   const bool cut = bid >= nfull;
-  const int u = cut ? bid - nfull : 0, nparts = cut ? nsplit : 1, part = u % nparts;
-  const long long col = col0 + (cut ? nfull + u / nparts : bid);
+  const int u0 = cut ? bid - nfull : 0, nparts = cut ? nsplit : 1, part = u0 % nparts;
+  const long long col = col0 + (cut ? nfull + u0 / nparts : bid);
   const int wlo = part * g.ncz / nparts, whi = (part + 1) * g.ncz / nparts - 1;
   const int zlo = tab.corners[2][wlo], zhi = tab.corners[2][whi] + g.pz - 1;  // its planes
   const int ci = (int)(col / g.ncy), cj = (int)(col % g.ncy);
   const int cx = tab.corners[0][ci], cy = tab.corners[1][cj];
-  const int tid = threadIdx.x;
-  const int blk = tid / ks, kq = tid - (tid / ks) * ks;
+  const int tid = threadIdx.x, lane = tid & 31;
+  const int kq = lane / BW, blk = (tid >> 5) * BW + (lane & (BW - 1));
   const bool owner = blk < nblk;
   int bi = 0, bj = 0;
   if (owner) {
     int rem = blk;
-    while (bi < nb && rem >= nb - bi) {
+    while (rem >= nb - bi) {
       rem -= nb - bi;
       ++bi;
     }
     bj = bi + rem;
   }
-  constexpr int ucount = 16 / ks;  // window entries this thread updates: [kq * ucount, kq * ucount + ucount)
+  // quads of the block's rows and columns (an absent one reads the last quad;
+  // what comes of it is not stored)
+  const int qa0 = bi, qa1 = min(bi + nb, nq - 1), qb0 = bj, qb1 = min(bj + nb, nq - 1);
   const uint32_t plane_bytes = (uint32_t)(rows * T * sizeof(float));
+  auto fetch = [&](int z, int slot) {  // plane z into a slot that nothing reads or fills
+    mbar_expect_tx(bar0 + 8 * slot, plane_bytes);
+    tma_load_4d((uint32_t)__cvta_generic_to_shared(smz + slot * pf), xmap, bar0 + 8 * slot, 0, z, cy, cx);
+  };
 
-  for (int e = tid; e < ring * 16 * nblk; e += nthreads) win[e] = 0.f;
+  for (int e = tid; e < ring * 16 * nblk; e += nthreads) win[e] = make_float4(0.f, 0.f, 0.f, 0.f);
   if (tid == 0) {
     mbar_init(bar0, 1);
-    mbar_init(bar1, 1);
+    mbar_init(bar0 + 8, 1);
     asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
   }
   __syncthreads();
-  if (tid == 0 && zlo <= zhi) {
-    mbar_expect_tx(bar0, plane_bytes);
-    tma_load_4d((uint32_t)__cvta_generic_to_shared(plane0), xmap, bar0, 0, zlo, cy, cx);
-  }
+  if (tid == 0 && zlo <= zhi) fetch(zlo, 0);
   float* G0 = gram + (size_t)((col - col0) * g.ncz) * T * T;
-  int gave_up = 0;  // uniform: a wait of some thread gave up at plane stop_z
-  int stop_z = zhi;
-  bool own_wait_ok = true;
-  for (int z = zlo; z <= zhi && !gave_up; ++z) {
-    const int it = z - zlo, slot = it & 1;
+  const bool aligned = (reinterpret_cast<uintptr_t>(gram) & 15) == 0;  // a caller's block may not be
+  float2 acc[8][4];  // row u of the block, column pairs
+#pragma unroll
+  for (int u = 0; u < 8; ++u)
+#pragma unroll
+    for (int v = 0; v < 4; ++v) acc[u][v] = make_float2(0.f, 0.f);
+  int nlo = tab.cover[2][2 * zlo], nhi = tab.cover[2][2 * zlo + 1];
+  for (int z = zlo; z <= zhi; ++z) {
+    const int slot = (z - zlo) & 1;
     // Each slot's barrier has at most one phase pending: plane z + 1 goes into
     // the slot whose previous plane (z - 1) every thread waited for in full.
-    const bool issued_next = z + 1 <= zhi;
-    if (tid == 0 && issued_next) {
-      const uint32_t nb_ = slot ? bar0 : bar1;
+    if (tid == 0 && z < zhi) {
       asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
-      mbar_expect_tx(nb_, plane_bytes);
-      tma_load_4d((uint32_t)__cvta_generic_to_shared(slot ? plane0 : plane1), xmap, nb_, 0, z + 1, cy, cx);
+      fetch(z + 1, slot ^ 1);
     }
-    const bool ok = mbar_wait_bounded(slot ? bar1 : bar0, (uint32_t)((it >> 1) & 1), status);
-    const int klo = max(tab.cover[2][2 * z], wlo), khi = min(tab.cover[2][2 * z + 1], whi);
+    // the column's windows holding plane z, and this unit's among them; the next
+    // plane's are fetched here
+    const int clo = nlo, chi = nhi;
+    if (z < zhi) {
+      nlo = tab.cover[2][2 * z + 2];
+      nhi = tab.cover[2][2 * z + 3];
+    }
+    const int klo = max(clo, wlo), khi = min(chi, whi);
+    const uint32_t parity = ((z - zlo) >> 1) & 1;
+    const bool ok = mbar_wait_bounded(bar0 + 8 * slot, parity, status);
     if (klo <= khi) {
-      const float* pl = slot ? plane1 : plane0;
-      float acc[16];
+      const float4* row = reinterpret_cast<const float4*>(smz + slot * pf) + kq * nq;
+      auto add_row = [&]() {
+        const float4 a0 = row[qa0], a1 = row[qa1], b0 = row[qb0], b1 = row[qb1];
+        const float av[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
+        const float2 bv[4] = {{b0.x, b0.y}, {b0.z, b0.w}, {b1.x, b1.y}, {b1.z, b1.w}};
 #pragma unroll
-      for (int u = 0; u < 16; ++u) acc[u] = 0.f;
-      const float4* rp = reinterpret_cast<const float4*>(pl);
-      const int ld4 = T >> 2;
-#pragma unroll 4
-      for (int r = kq; r < rows; r += ks) {
-        const float4 va = rp[r * ld4 + bi];
-        const float4 vb = rp[r * ld4 + bj];
-        const float a4[4] = {va.x, va.y, va.z, va.w};
-        const float b4[4] = {vb.x, vb.y, vb.z, vb.w};
+        for (int u = 0; u < 8; ++u)
 #pragma unroll
-        for (int u = 0; u < 4; ++u)
-#pragma unroll
-          for (int v = 0; v < 4; ++v) acc[u * 4 + v] = fmaf(a4[u], b4[v], acc[u * 4 + v]);
+          for (int v = 0; v < 4; ++v) fma2(acc[u][v], make_float2(av[u], av[u]), bv[v]);
+        row += KS * nq;
+      };
+      // (the same number of rows for every lane, then the remainder)
+#pragma unroll 2
+      for (int i = rows / KS; i > 0; --i) add_row();
+      if (kq < rows % KS) add_row();
+    }
+    // this slot is refilled by the copy issued at the start of the next iteration
+    if (__syncthreads_or(!ok)) {
+      // A wait gave up: nothing more is issued; thread 0 waits (bounded) for the
+      // copies still in flight - this plane if its own wait gave up, and the next -
+      // so that none lands after the CTA's shared memory is freed.
+      if (tid == 0) {
+        if (!ok) mbar_wait_bounded(bar0 + 8 * slot, parity, status);
+        if (z < zhi) mbar_wait_bounded(bar0 + 8 * (slot ^ 1), ((z + 1 - zlo) >> 1) & 1, status);
       }
-      // combine the ks partial sums (every lane of the group ends with the total)
-      if (ks >= 2) {
+      return;
+    }
+    if (klo > khi) continue;
+    // Planes in the same windows are summed together; the sum goes to the
+    // windows at the last of them (a window starts and ends at such a break).
+    if (z < zhi && nlo == clo && nhi == chi) continue;
+    // halving exchanges over the KS lanes of a block: each step a lane keeps half
+    // of its rows and adds its partner's copies of them
+    float2 mine[NR][4];
+    {
+      float2 h4[4][4], h2[2][4];
 #pragma unroll
-        for (int u = 0; u < 16; ++u) acc[u] += __shfl_xor_sync(0xffffffffu, acc[u], 1);
-      }
-      if (ks >= 4) {
+      for (int u = 0; u < 4; ++u)
 #pragma unroll
-        for (int u = 0; u < 16; ++u) acc[u] += __shfl_xor_sync(0xffffffffu, acc[u], 2);
-      }
-      if (owner) {
-        // this thread's entries of the 4x4 block, e = kq * ucount + q
-        float mine[ucount];
-#pragma unroll
-        for (int q = 0; q < ucount; ++q) {
-          float v = acc[q];
-#pragma unroll
-          for (int c = 1; c < ks; ++c)
-            if (kq == c) v = acc[c * ucount + q];
-          mine[q] = v;
+        for (int v = 0; v < 4; ++v) {
+          const bool hi = kq >= KS / 2;
+          const float2 keep = hi ? acc[u + 4][v] : acc[u][v], send = hi ? acc[u][v] : acc[u + 4][v];
+          h4[u][v].x = keep.x + __shfl_xor_sync(0xffffffffu, send.x, 16);
+          h4[u][v].y = keep.y + __shfl_xor_sync(0xffffffffu, send.y, 16);
         }
-        // Windows are consecutive and their corners increase, so only the
-        // lowest window holding plane z (klo) can end at z.
-        const bool klo_ends = z == tab.corners[2][klo] + g.pz - 1;
-        int slot = klo % ring;
-        for (int k = klo; k <= khi; ++k) {
-          float* w = win + (size_t)slot * 16 * nblk + blk + (size_t)kq * ucount * nblk;
-          if (k != klo || !klo_ends) {
+      if constexpr (KS == 2) {
 #pragma unroll
-            for (int q = 0; q < ucount; ++q) w[q * nblk] += mine[q];
-          } else {
-            float* G = G0 + (size_t)k * T * T;
+        for (int u = 0; u < NR; ++u)
 #pragma unroll
-            for (int q = 0; q < ucount; ++q) {
-              const int e = kq * ucount + q;
-              const float val = w[q * nblk] + mine[q];
-              w[q * nblk] = 0.f;
-              const int r = bi * 4 + (e >> 2), c = bj * 4 + (e & 3);
-              G[(size_t)r * T + c] = val;
-              G[(size_t)c * T + r] = val;
+          for (int v = 0; v < 4; ++v) mine[u][v] = h4[u][v];
+      } else {
+#pragma unroll
+        for (int u = 0; u < 2; ++u)
+#pragma unroll
+          for (int v = 0; v < 4; ++v) {
+            const bool hi = (lane >> 3) & 1;
+            const float2 keep = hi ? h4[u + 2][v] : h4[u][v], send = hi ? h4[u][v] : h4[u + 2][v];
+            h2[u][v].x = keep.x + __shfl_xor_sync(0xffffffffu, send.x, 8);
+            h2[u][v].y = keep.y + __shfl_xor_sync(0xffffffffu, send.y, 8);
+          }
+        if constexpr (KS == 4) {
+#pragma unroll
+          for (int u = 0; u < NR; ++u)
+#pragma unroll
+            for (int v = 0; v < 4; ++v) mine[u][v] = h2[u][v];
+        } else {
+#pragma unroll
+          for (int v = 0; v < 4; ++v) {
+            const bool hi = (lane >> 2) & 1;
+            const float2 keep = hi ? h2[1][v] : h2[0][v], send = hi ? h2[0][v] : h2[1][v];
+            mine[0][v].x = keep.x + __shfl_xor_sync(0xffffffffu, send.x, 4);
+            mine[0][v].y = keep.y + __shfl_xor_sync(0xffffffffu, send.y, 4);
+          }
+        }
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < 8; ++u)
+#pragma unroll
+      for (int v = 0; v < 4; ++v) acc[u][v] = make_float2(0.f, 0.f);
+    if (!owner) continue;
+    // Windows are consecutive and their corners increase, so only the lowest
+    // window holding plane z (klo) can end at z.
+    const bool klo_ends = z == tab.corners[2][klo] + g.pz - 1;
+    int wslot = klo % ring;
+    for (int k = klo; k <= khi; ++k) {
+      float4* w = win + (size_t)wslot * 16 * nblk + kq * nblk + blk;
+      const bool ends = k == klo && klo_ends;
+      float* G = G0 + (size_t)k * T * T;
+#pragma unroll
+      for (int u = 0; u < NR; ++u)
+#pragma unroll
+        for (int cq = 0; cq < 2; ++cq) {  // the row's two column quads
+          float4 v = w[(2 * u + cq) * nown];
+          v.x += mine[u][2 * cq].x;
+          v.y += mine[u][2 * cq].y;
+          v.z += mine[u][2 * cq + 1].x;
+          v.w += mine[u][2 * cq + 1].y;
+          w[(2 * u + cq) * nown] = ends ? make_float4(0.f, 0.f, 0.f, 0.f) : v;
+          const int ub = kq * NR + u;  // row of the block
+          const int fr = ub < 4 ? 4 * bi + ub : 4 * (bi + nb) + ub - 4, qc = cq ? bj + nb : bj;
+          if (ends && fr < T && qc < nq) {
+            float* gr = G + (size_t)fr * T + 4 * qc;
+            if (aligned) {
+              *reinterpret_cast<float4*>(gr) = v;
+            } else {
+              gr[0] = v.x;
+              gr[1] = v.y;
+              gr[2] = v.z;
+              gr[3] = v.w;
+            }
+            if (bi != bj) {
+              float* gc = G + (size_t)(4 * qc) * T + fr;
+              gc[0] = v.x;
+              gc[T] = v.y;
+              gc[2 * (size_t)T] = v.z;
+              gc[3 * (size_t)T] = v.w;
             }
           }
-          if (++slot == ring) slot = 0;
         }
-      }
+      if (++wslot == ring) wslot = 0;
     }
-    // this slot is refilled by the TMA issued at the start of the next iteration
-    gave_up = __syncthreads_or(!ok);
-    stop_z = z;
-    own_wait_ok = ok;
-  }
-  if (gave_up && tid == 0) {
-    // a wait gave up: nothing more was issued; wait (bounded) for the copies
-    // still in flight - plane stop_z if this thread's own wait gave up, and
-    // plane stop_z + 1 - so that none lands after the CTA's shared memory is freed
-    const int it = stop_z - zlo, slot = it & 1;
-    drain_copies(!own_wait_ok, slot ? bar1 : bar0, (uint32_t)((it >> 1) & 1), stop_z + 1 <= zhi,
-                 slot ? bar0 : bar1, (uint32_t)(((it + 1) >> 1) & 1), status);
   }
 }
 
+// (T <= 128 needs at most 544 threads at KS = 4, 288 at KS = 2; KS = 8 runs up to T = 88)
+constexpr int kGramzMaxThreads = 512;
+
 template <int KS>
-__global__ void __maxnreg__(64) gram_z_kernel(const __grid_constant__ CUtensorMap xmap, float* __restrict__ gram, Geom g,
-                              AxisTables tab, long long col0, int ring, int nfull, int nsplit,
-                              int* status) {
+__global__ void __maxnreg__(128)
+    gram_z_kernel(const __grid_constant__ CUtensorMap xmap, float* __restrict__ gram, Geom g, AxisTables tab,
+                  long long col0, int ring, int nfull, int nsplit, int* status) {
   gram_z_body<KS>(&xmap, gram, g, tab, col0, ring, nfull, nsplit, status, (int)blockIdx.x);
 }
 

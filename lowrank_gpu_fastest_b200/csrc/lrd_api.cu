@@ -52,6 +52,8 @@ int cuda_fail(cudaError_t err, const char* what) {
     if (e_ != cudaSuccess) return cuda_fail(e_, #call);  \
   } while (0)
 
+constexpr size_t kSmemMax = 227 * 1024;  // dynamic shared memory of one CTA
+
 size_t align256(size_t x) { return (x + 255) & ~size_t(255); }
 
 // Sorted corner positions along one axis (common.py:40-43):
@@ -80,8 +82,10 @@ struct lrd_plan {
   bool use_gramtc;         // the column Gram on tcgen05 (tensor forms)
   bool gramtc_bf16 = false; // ... with BF16 3-term split operands instead of 3xTF32
   size_t smem_gramtc;
-  int gramz_ring;          // window accumulator slots
-  int gramz_ks = 1;        // voxel-row split per 4x4 Gram block (threads per block)
+  int gramz_ring;          // window accumulator slots of the column Gram
+  int gramz_cut = 1;       // window ranges every column is cut into (> 1: the full ring does not fit)
+  int gramtc_ring = 1;     // ... of the tensor-core column Gram (always the full ring)
+  int gramz_ks = 4;        // voxel-row split per 8x8 Gram block (threads per block)
   bool eigh_cta = false;   // eigensolver: one CTA per matrix (else one warp)
   size_t smem_gramz;
   int gramz_slots = 0;     // column CTAs resident at once on the device (0: never cut columns)
@@ -138,12 +142,14 @@ constexpr long long kIoSlabBytes = 7ll << 19;
 
 namespace {
 
-// Voxel-row split of the column Gram. Measured on B200 (96x96x48xT, 11^3,
-// stride 3, before short last waves were cut into window ranges): T = 48
-// runs 0.80 ms with 2 threads per block (160-thread CTAs)
-// against 0.96 ms unsplit and 1.27 ms with 4; T = 32, 64 and 96 are fastest
-// unsplit (0.58 / 1.44 / 1.21 ms, the split costing 30-60%).
-int gramz_split(int T) { return (T > 40 && T <= 56) ? 2 : 1; }
+// Voxel-row split of the column Gram (threads per 8 x 8 block). Measured on
+// B200, Gram phase ms with 2 / 4 / 8: 96x96x48x48, 11^3, stride 3 0.80 / 0.52 /
+// 0.52 (48x48x24x48 0.125 / 0.097 / 0.090: 8 there); 96x96x48x32, 5^3, stride 1
+// 1.77 / 1.40 / 1.69; 101x87x43x64, 7^3, stride 2 1.17 / 0.98 / 1.50;
+// 64x64x48x96, 11^3, stride 3 0.90 / 0.70 / -. A CTA of fewer than 48 threads at
+// 4 (T <= 24) takes 8. The split does not depend on the launch: it changes the
+// rounding.
+int gramz_split(int T) { return (T <= 24 || (T > 40 && T <= 56)) ? 8 : 4; }
 
 void* gramtc_kernel_ptr(bool bf16) {
   return bf16 ? (void*)lrd::gram_tc_kernel<true> : (void*)lrd::gram_tc_kernel<false>;
@@ -152,8 +158,8 @@ void* gramtc_kernel_ptr(bool bf16) {
 void* gramz_kernel_ptr(int ks) {
   switch (ks) {
     case 2: return (void*)lrd::gram_z_kernel<2>;
-    case 4: return (void*)lrd::gram_z_kernel<4>;
-    default: return (void*)lrd::gram_z_kernel<1>;
+    case 8: return (void*)lrd::gram_z_kernel<8>;
+    default: return (void*)lrd::gram_z_kernel<4>;
   }
 }
 
@@ -339,6 +345,8 @@ int set_smem(const void* fn, size_t bytes) {
   if (bytes <= cur) return LRD_OK;
   e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
   if (e != cudaSuccess) return cuda_fail(e, "cudaFuncSetAttribute(max dynamic smem)");
+  e = cudaFuncSetAttribute(fn, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+  if (e != cudaSuccess) return cuda_fail(e, "cudaFuncSetAttribute(shared memory carveout)");
   cur = bytes;
   return LRD_OK;
 }
@@ -398,11 +406,11 @@ int encode_plane_map(const lrd_plan* P, const float* xc, CUtensorMap* map) {
 
 // Gram matrices of the patch columns [col_lo, col_hi) (x-major column index
 // ci * ncy + cj; -1 = all), i.e. of patches [col_lo * ncz, col_hi * ncz).
-// ``spread``: a launch of fewer columns than the device holds at once has all
-// of them cut into window ranges (more, shorter CTAs: lower latency for more
-// plane reads, for a Gram on the critical path of an otherwise idle device).
+// ``spread``: a launch of fewer columns than half of what the device holds at once
+// has all of them cut into window ranges (more, shorter CTAs: lower latency for
+// more plane reads, for a Gram on the critical path of an otherwise idle device).
 int run_gram(const lrd_plan* P, char* ws, float* d_gram, cudaStream_t st, long long col_lo = 0,
-             long long col_hi = -1, bool spread = false) {
+             long long col_hi = -1, bool spread = true) {
   const float* xc = reinterpret_cast<const float*>(ws + P->off_xc);
   const long long ncol = (long long)P->g.ncx * P->g.ncy;
   if (col_hi < 0) col_hi = ncol;
@@ -420,10 +428,11 @@ int run_gram(const lrd_plan* P, char* ws, float* d_gram, cudaStream_t st, long l
       // they finish: cut those columns into window ranges instead.
       const long long slots = P->use_gramtc ? P->gramtc_slots : P->gramz_slots;
       long long nfull = nc;
-      int nsplit = 1;
+      const int cut = P->use_gramtc ? 1 : P->gramz_cut;  // ranges a column must be cut into
+      int nsplit = cut;
       const long long rem = slots > 0 ? nc % slots : 0;
-      if (spread && slots > 0 && nc < slots && P->g.ncz > 1) {
-        nsplit = (int)std::min<long long>(P->g.ncz, std::max<long long>(1, slots / nc));
+      if (cut > 1 || (spread && slots > 0 && nc < slots && P->g.ncz > 1)) {
+        if (spread && slots > 0) nsplit = (int)std::min<long long>(P->g.ncz, std::max<long long>(cut, slots / nc));
         if (nsplit > 1) nfull = 0;
         else nsplit = 1;
       } else if (slots > 0 && nc > slots && rem > 0 && 2 * rem <= slots && P->g.ncz > 1) {
@@ -435,10 +444,10 @@ int run_gram(const lrd_plan* P, char* ws, float* d_gram, cudaStream_t st, long l
       if (P->use_gramtc) {
         if (P->gramtc_bf16)
           lrd::gram_tc_kernel<true><<<(unsigned)grid, lrd::kGramTcThreads, P->smem_gramtc, st>>>(
-              map, d_gram + c0 * P->g.ncz * TT, P->g, P->tab, c0, P->gramz_ring, (int)nfull, nsplit, status);
+              map, d_gram + c0 * P->g.ncz * TT, P->g, P->tab, c0, P->gramtc_ring, (int)nfull, nsplit, status);
         else
           lrd::gram_tc_kernel<false><<<(unsigned)grid, lrd::kGramTcThreads, P->smem_gramtc, st>>>(
-              map, d_gram + c0 * P->g.ncz * TT, P->g, P->tab, c0, P->gramz_ring, (int)nfull, nsplit, status);
+              map, d_gram + c0 * P->g.ncz * TT, P->g, P->tab, c0, P->gramtc_ring, (int)nfull, nsplit, status);
         rc = launch_check("gram_tc_kernel launch");
       } else {
         void* fn = gramz_kernel_ptr(P->gramz_ks);
@@ -790,10 +799,16 @@ int create_plan(const lrd_problem* pr, const std::vector<int32_t>* x_corners, lr
   {
     int ring = 1;
     for (int z = 0; z < pr->nz; ++z) ring = std::max(ring, cover[2][2 * z + 1] - cover[2][2 * z] + 1);
+    P->gramtc_ring = ring;
+    P->gramz_ks = pr->gram_split > 0 ? 2 * pr->gram_split : gramz_split(T);
+    while (P->gramz_ks > 2 && lrd::gramz_threads(T, P->gramz_ks) > lrd::kGramzMaxThreads) P->gramz_ks /= 2;
+    // The window ring, or the part of it that fits beside the planes (the
+    // columns are then cut into ranges of that many windows).
     P->gramz_ring = ring;
-    P->gramz_ks = pr->gram_split > 0 ? pr->gram_split : gramz_split(T);
-    P->smem_gramz = lrd::gramz_smem_bytes(pr->px * pr->py, T, ring, P->gram_threads);
-    P->use_gramz = (T % 4 == 0) && P->smem_gramz <= 200 * 1024 && tensor_map_encoder() != nullptr &&
+    while (P->gramz_ring > 1 && lrd::gramz_smem_bytes(pr->px, pr->py, T, P->gramz_ring) > kSmemMax) --P->gramz_ring;
+    P->gramz_cut = P->gramz_ring < ring ? (g.ncz + P->gramz_ring - 1) / P->gramz_ring : 1;
+    P->smem_gramz = lrd::gramz_smem_bytes(pr->px, pr->py, T, P->gramz_ring);
+    P->use_gramz = (T % 4 == 0) && P->smem_gramz <= kSmemMax && tensor_map_encoder() != nullptr &&
                    pr->px <= 256 && pr->py <= 256;
     P->gramtc_bf16 = pr->form == LRD_FORM_TENSOR_BF16;
     P->smem_gramtc = lrd::gramtc_smem_bytes(pr->px * pr->py, T, ring, P->gramtc_bf16);
@@ -1050,7 +1065,7 @@ int run_pipelined(const lrd_plan* P, const float* d_vol, float* d_out, char* ws,
       return rc;
     LRD_CUDA(cudaEventRecord(ev(s, 1), prep));
     planes_in = std::max(planes_in, x_need);
-    if ((rc = run_gram(P, ws, gv, prep, ci_done * colz, ci_end * colz))) return rc;
+    if ((rc = run_gram(P, ws, gv, prep, ci_done * colz, ci_end * colz, false))) return rc;
     LRD_CUDA(cudaEventRecord(ev(s, 2), prep));
     // successive slabs' solves on two streams: one slab's solve takes a matrix's
     // latency however few matrices it has, so two run side by side
