@@ -262,6 +262,10 @@ size_t eigh_smem_for(int T, bool cta) {
   if (T <= 48) return lrd::eigh_reg_smem_floats<48>();
   return lrd::eigh_reg_smem_floats<64>();
 }
+int eigh_mats_for(int T, bool cta) {
+  if (cta || T > 48) return 1;
+  return T <= 32 ? lrd::eigh_reg_mats<32>() : lrd::eigh_reg_mats<48>();
+}
 const void* eigh_kernel_for(int T, bool cta, unsigned* threads = nullptr) {
   if (threads) *threads = cta ? (T <= 64 ? 64u : (T <= 96 ? 96u : 128u)) : 32u;
   if (cta) {
@@ -512,11 +516,13 @@ int run_eigh(const lrd_plan* P, char* ws, const float* d_gram, float* d_vecs, fl
     const int nv = P->g.nvox_patch;
     unsigned eth = 32;
     const void* efn = eigh_kernel_for(T, P->eigh_cta, &eth);
+    long long nmat = nb;
+    const long long mats = eigh_mats_for(T, P->eigh_cta);  // matrices per block
     long long p0v = p0;
     int tv = T, nvv = nv;
     void* eargs[] = {(void*)&gin, (void*)&vout, (void*)&lout, (void*)&r,      (void*)&w,   (void*)&s2,
-                     (void*)&tv,  (void*)&nvv,  (void*)&p0v,  (void*)&rcount, (void*)&rids};
-    cudaError_t le = cudaLaunchKernel(efn, dim3((unsigned)nb), dim3(eth), eargs, P->smem_eigh, st);
+                     (void*)&tv,  (void*)&nvv,  (void*)&p0v,  (void*)&rcount, (void*)&rids, (void*)&nmat};  // nmat: the warp kernels
+    cudaError_t le = cudaLaunchKernel(efn, dim3((unsigned)((nb + mats - 1) / mats)), dim3(eth), eargs, P->smem_eigh, st);
     if (le != cudaSuccess) return cuda_fail(le, "eigh kernel launch");
     int rc = launch_check("eigh kernel launch");
     if (rc) return rc;
