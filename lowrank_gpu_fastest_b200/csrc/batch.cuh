@@ -120,15 +120,15 @@ __global__ void __launch_bounds__(kRefineThreads)
                    (int)(blockIdx.x - off[i]), (int)(off[i + 1] - off[i]));
 }
 
-template <int Q, bool ACCURATE>
-__global__ void __launch_bounds__(32 * kReconWarps)
+template <int T, bool ACCURATE>
+__global__ void __launch_bounds__(32 * kReconWarps, recon_warp_ctas<T, ACCURATE>())
     recon_warp_batch_kernel(const BatchVol* __restrict__ vols, const int* __restrict__ list,
                             const long long* __restrict__ off, int n) {
   const int i = batch_find(off, n, blockIdx.x);
   const BatchVol& V = vols[list[i]];
   const SlabIO io{0, V.g.nx, 0, nullptr, V.g.nx, nullptr};
-  recon_warp_body<Q, ACCURATE>(V.xc, V.mean, V.gv, V.rank, V.wgt, V.out, V.g, V.tab, 0, io,
-                               (int)(blockIdx.x - off[i]));
+  recon_warp_body<T, ACCURATE>(V.xc, V.mean, V.gv, V.rank, V.wgt, V.out, V.g, V.tab, 0, io,
+                               V.status, (int)(blockIdx.x - off[i]));
 }
 
 // Ranks of every listed volume that asked for them, into its rank array.

@@ -47,7 +47,6 @@
 #pragma once
 
 #include "eigh.cuh"
-#include "gram_z.cuh"  // fma2
 
 namespace lrd {
 
@@ -59,11 +58,6 @@ __device__ long long* g_phase_clocks;  // 8 stamps per block, set by a probe bui
 #define LRD_STAMP(i) \
   do { } while (0)
 #endif
-
-template <int V>
-struct IntTag {
-  static constexpr int value = V;
-};
 
 // Lanes per matrix and matrices per warp (= per block).
 template <int TMAX>
@@ -143,25 +137,6 @@ __device__ __forceinline__ void sub_allsum(float2 (&v)[G]) {
     v[i].x = __shfl_sync(0xffffffffu, f[0], (2 * i) * (L / N), L);
     v[i].y = __shfl_sync(0xffffffffu, f[0], (2 * i + 1) * (L / N), L);
   }
-}
-
-__device__ __forceinline__ float2 add2(float2 a, float2 b) {
-  unsigned long long ra, rb, rc;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(ra) : "f"(a.x), "f"(a.y));
-  asm("mov.b64 %0, {%1, %2};" : "=l"(rb) : "f"(b.x), "f"(b.y));
-  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(rc) : "l"(ra), "l"(rb));
-  float2 c;
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(c.x), "=f"(c.y) : "l"(rc));
-  return c;
-}
-__device__ __forceinline__ float2 mul2(float2 a, float2 b) {
-  unsigned long long ra, rb, rc;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(ra) : "f"(a.x), "f"(a.y));
-  asm("mov.b64 %0, {%1, %2};" : "=l"(rb) : "f"(b.x), "f"(b.y));
-  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(rc) : "l"(ra), "l"(rb));
-  float2 c;
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(c.x), "=f"(c.y) : "l"(rc));
-  return c;
 }
 
 // Sturm counts: c[j] = sign changes of the sequence at x[j] = eigenvalues below
@@ -279,95 +254,80 @@ __device__ __forceinline__ void bisect_reg(const float* d, const float* e, float
     co[i] = make_float4(di, di, -e2, -e2);
   }
   __syncwarp();
+  // [clo, chi): the eigenvalues between the ends, j among them; they all have this
+  // interval
   float lo[C], hi[C], x[C];
-  int c[C], start[C], m[C];
+  int clo[C], chi[C], c[C];
 #pragma unroll
   for (int k = 0; k < C; ++k) {
     lo[k] = glo;
     hi[k] = ghi;
+    clo[k] = 0;
+    chi[k] = n;
   }
-  // Both matrices of a warp take part in every round, but what happens to one
-  // depends on itself alone: a matrix that is done keeps its intervals.
-  const unsigned half = L == 32 ? 0xffffffffu : ((1u << (L & 31)) - 1u) << sh;
-  bool shared = true;  // some interval of this matrix holds several eigenvalues
+  // The matrices of a warp go through the rounds together; what happens to one
+  // depends on itself alone (one that is done keeps its intervals).
+  constexpr unsigned field = L == 32 ? 0xffffffffu : (1u << (L & 31)) - 1u;
   for (int it = 0; it < 200; ++it) {
-    bool run = false;
+    bool run = false, several = false;
 #pragma unroll
     for (int k = 0; k < C; ++k) {
+      const int j = l + L * k;
       const float tol = fmaxf(abstol, 2.f * eps * fmaxf(fabsf(lo[k]), fabsf(hi[k])));
       const float mid = 0.5f * (lo[k] + hi[k]);
-      run |= l + L * k < n && hi[k] - lo[k] > tol && mid > lo[k] && mid < hi[k];
+      run |= j < n && hi[k] - lo[k] > tol && mid > lo[k] && mid < hi[k];
+      several |= j < n && chi[k] - clo[k] > 1;
+      x[k] = mid;
     }
     const unsigned running = __ballot_sync(0xffffffffu, run);
     if (running == 0) break;
-    const bool on = running & half;
-    const bool any_shared = __any_sync(0xffffffffu, shared && on);
-    if (any_shared) {
-      // the first eigenvalue of each interval, as a bit mask over j
-      unsigned long long starts = 0;
+    const bool on = (running >> (sh & 31)) & field;
+    const bool any_several = __any_sync(0xffffffffu, several && on);
+    if (any_several) {
 #pragma unroll
       for (int k = 0; k < C; ++k) {
-        float plo = __shfl_up_sync(0xffffffffu, lo[k], 1, L), phi = __shfl_up_sync(0xffffffffu, hi[k], 1, L);
-        if (k > 0) {
-          const float qlo = __shfl_sync(0xffffffffu, lo[k > 0 ? k - 1 : 0], L - 1, L);
-          const float qhi = __shfl_sync(0xffffffffu, hi[k > 0 ? k - 1 : 0], L - 1, L);
-          if (l == 0) {
-            plo = qlo;
-            phi = qhi;
-          }
-        }
-        const bool first = (k == 0 && l == 0) || plo != lo[k] || phi != hi[k] || l + L * k >= n;
-        const unsigned b = __ballot_sync(0xffffffffu, first);
-        const unsigned mine = L == 32 ? b : (b >> sh) & ((1u << (L & 31)) - 1u);
-        starts |= (unsigned long long)mine << (L * k);
+        const int m = chi[k] - clo[k];
+        if (m > 1)
+          x[k] = fmaf(hi[k] - lo[k], __fdividef((float)(l + L * k - clo[k] + 1), (float)(m + 1)), lo[k]);
       }
-      bool more = false;
-#pragma unroll
-      for (int k = 0; k < C; ++k) {
-        const int j = l + L * k;
-        start[k] = 63 - __clzll(starts & (~0ull >> (63 - j)));
-        const unsigned long long after = j < 63 ? starts >> (j + 1) : 0ull;
-        const int end = after ? j + __ffsll(after) : C * L;
-        m[k] = max(1, min(end, n) - start[k]);
-        more |= m[k] > 1;
-        x[k] = m[k] == 1 ? 0.5f * (lo[k] + hi[k])
-                         : lo[k] + (hi[k] - lo[k]) * __fdividef((float)(j - start[k] + 1), (float)(m[k] + 1));
-      }
-      shared = __ballot_sync(0xffffffffu, more) & half;
-    } else {
-#pragma unroll
-      for (int k = 0; k < C; ++k) x[k] = 0.5f * (lo[k] + hi[k]);
     }
     sturm_counts<C>(co, n16, x, c);
-    if (any_shared) {
-      __syncwarp();  // the previous round's readers are done
+    if (any_several) {
 #pragma unroll
       for (int k = 0; k < C; ++k) {
         px[l + L * k] = x[k];
         cnt[l + L * k] = c[k];
       }
       __syncwarp();
+    }
+    if (on) {
 #pragma unroll
       for (int k = 0; k < C; ++k) {
         const int j = l + L * k;
-        if (j < n && on) {
+        if (chi[k] - clo[k] > 1 && j < n) {
           // first point of the interval with more than j eigenvalues below it
-          int a = start[k], b = start[k] + m[k];
+          const int p0 = clo[k], p1 = chi[k];
+          int a = p0, b = p1;
           while (a < b) {
             const int mid = (a + b) >> 1;
             if (cnt[mid] > j) b = mid; else a = mid + 1;
           }
-          if (a > start[k]) lo[k] = px[a - 1];
-          if (a < start[k] + m[k]) hi[k] = px[a];
+          if (a > p0) {
+            lo[k] = px[a - 1];
+            clo[k] = max(clo[k], cnt[a - 1]);
+          }
+          if (a < p1) {
+            hi[k] = px[a];
+            chi[k] = min(chi[k], cnt[a]);
+          }
+        } else if (c[k] > j) {
+          hi[k] = x[k];
+        } else {
+          lo[k] = x[k];
         }
       }
-    } else {
-#pragma unroll
-      for (int k = 0; k < C; ++k) {
-        if (on && c[k] > l + L * k) hi[k] = x[k];
-        if (on && c[k] <= l + L * k) lo[k] = x[k];
-      }
     }
+    if (any_several) __syncwarp();  // the next round's points go to the same place
   }
 #pragma unroll
   for (int k = 0; k < C; ++k)

@@ -122,16 +122,6 @@ __host__ __device__ inline size_t gramz_smem_bytes(int px, int py, int T, int ri
   return sizeof(float) * (2 * gramz_plane_floats(px * py, T) + (size_t)ring * 64 * gramz_nblk(T)) + 2 * sizeof(uint64_t);
 }
 
-// (c0, c1) += (a, a) * (b0, b1): two IEEE FMAs in one instruction.
-__device__ __forceinline__ void fma2(float2& c, float2 a, float2 b) {
-  unsigned long long ra, rb, rc;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(ra) : "f"(a.x), "f"(a.y));
-  asm("mov.b64 %0, {%1, %2};" : "=l"(rb) : "f"(b.x), "f"(b.y));
-  asm("mov.b64 %0, {%1, %2};" : "=l"(rc) : "f"(c.x), "f"(c.y));
-  asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(rc) : "l"(ra), "l"(rb));
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(c.x), "=f"(c.y) : "l"(rc));
-}
-
 // grid: nfull + (columns - nfull) * nsplit CTAs; block: gramz_threads(T, KS)
 // (T % 4 == 0, KS in {2, 4, 8}). CTA b < nfull computes every window of column
 // col0 + b; the columns after the first nfull are each cut into nsplit units

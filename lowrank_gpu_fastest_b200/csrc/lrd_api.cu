@@ -74,7 +74,7 @@ struct lrd_plan {
   long long nvox;
   int tpt;                 // recon frames per thread
   int split;               // recon threads per voxel
-  bool recon_warp = false; // reconstruction by recon_warp_kernel (2 x 2 x 2 voxels per warp)
+  bool recon_warp = false; // reconstruction by recon_warp_kernel
   bool recon_tc = false;   // reconstruction by recon_tc_kernel (tensor forms: 4 x 4 x 8 bricks on tcgen05)
   size_t smem_recon_tc = 0;
   int gram_threads;
@@ -316,10 +316,10 @@ void* recon_kernel_ptr(int tpt, int split, bool accurate) {
 
 void* recon_warp_ptr(int T, bool accurate) {
   switch (T) {
-    case 32: return accurate ? (void*)lrd::recon_warp_kernel<8, true> : (void*)lrd::recon_warp_kernel<8, false>;
-    case 48: return accurate ? (void*)lrd::recon_warp_kernel<12, true> : (void*)lrd::recon_warp_kernel<12, false>;
-    case 64: return accurate ? (void*)lrd::recon_warp_kernel<16, true> : (void*)lrd::recon_warp_kernel<16, false>;
-    case 96: return accurate ? (void*)lrd::recon_warp_kernel<24, true> : (void*)lrd::recon_warp_kernel<24, false>;
+    case 32: return accurate ? (void*)lrd::recon_warp_kernel<32, true> : (void*)lrd::recon_warp_kernel<32, false>;
+    case 48: return accurate ? (void*)lrd::recon_warp_kernel<48, true> : (void*)lrd::recon_warp_kernel<48, false>;
+    case 64: return accurate ? (void*)lrd::recon_warp_kernel<64, true> : (void*)lrd::recon_warp_kernel<64, false>;
+    case 96: return accurate ? (void*)lrd::recon_warp_kernel<96, true> : (void*)lrd::recon_warp_kernel<96, false>;
   }
   return nullptr;
 }
@@ -553,7 +553,7 @@ int run_recon(const lrd_plan* P, char* ws, float* d_out, cudaStream_t st, long l
   void* fn = P->recon_tc     ? recon_tc_ptr(P->g.nt)
              : P->recon_warp ? recon_warp_ptr(P->g.nt, acc)
                              : recon_kernel_ptr(P->tpt, P->split, acc);
-  const size_t smem = P->recon_tc ? P->smem_recon_tc : (P->recon_warp ? 0 : P->smem_recon);
+  const size_t smem = P->recon_tc ? P->smem_recon_tc : (P->recon_warp ? lrd::recon_warp_smem_bytes(P->g.nt) : P->smem_recon);
   lrd::Geom g = P->g;
   lrd::AxisTables tab = P->tab;
   int brick0 = (int)b_lo;
@@ -615,7 +615,7 @@ int validate_problem(const lrd_problem* pr) {
 // and the brick - the cost model's choice, or the problem's recon_split and
 // brick when set (a brick must fit the reconstruction kernel's threads per
 // CTA). Without either, frame counts the warp kernel is built for take it
-// (``warp``; brick 2 x 2 x recon_warp_bz(), four lanes per voxel).
+// (``warp``; recon_warp_brick()).
 // Measured on B200, reconstruction ms, 96x96x48x48 / 11^3 / stride 3:
 // brick kernel (3x3x3, 2 threads per voxel) 1.22 -> warp kernel (see DESIGN).
 int pick_layout(const lrd_problem* pr, const int dims[3], const int pat[3], const std::vector<int32_t> corners[3],
@@ -653,9 +653,7 @@ int pick_layout(const lrd_problem* pr, const int dims[3], const int pat[3], cons
     *warp = true;
     rsplit = 4;
     rtpt = pr->nt / 4;
-    best[0] = 2;
-    best[1] = 2;
-    best[2] = lrd::recon_warp_bz();
+    lrd::recon_warp_brick(pr->nt, pr->form != LRD_FORM_PLAIN, best);
     return LRD_OK;
   }
   pick_recon_layout(pr->nt, pr->recon_split, pr->form != LRD_FORM_PLAIN, rsplit, rtpt);
@@ -850,6 +848,7 @@ int create_plan(const lrd_problem* pr, const std::vector<int32_t>* x_corners, lr
     }
   }
   if (!rc) rc = set_smem(eigh_kernel_for(T, P->eigh_cta), P->smem_eigh);
+  if (!rc && P->recon_warp) rc = set_smem(recon_warp_ptr(T, pr->form != LRD_FORM_PLAIN), lrd::recon_warp_smem_bytes(T));
   if (!rc && !P->recon_tc) rc = set_smem(recon_kernel_ptr(P->tpt, P->split, false), P->smem_recon);
   if (!rc && !P->recon_tc) rc = set_smem(recon_kernel_ptr(P->tpt, P->split, true), P->smem_recon);
   if (!rc && P->recon_tc) rc = set_smem(recon_tc_ptr(T), P->smem_recon_tc);

@@ -43,4 +43,61 @@ __device__ __forceinline__ long long voxel_row(const Geom& g, int x, int y, int 
   return ((long long)x * g.ny + y) * g.nz + z;
 }
 
+// Packed float32 arithmetic: two IEEE operations in one instruction. c += a b. (A
+// mul2 may be contracted with an add2 of its result: see mul2_rn.)
+__device__ __forceinline__ void fma2(float2& c, float2 a, float2 b) {
+  unsigned long long ra, rb, rc;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(ra) : "f"(a.x), "f"(a.y));
+  asm("mov.b64 %0, {%1, %2};" : "=l"(rb) : "f"(b.x), "f"(b.y));
+  asm("mov.b64 %0, {%1, %2};" : "=l"(rc) : "f"(c.x), "f"(c.y));
+  asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(rc) : "l"(ra), "l"(rb));
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(c.x), "=f"(c.y) : "l"(rc));
+}
+
+__device__ __forceinline__ float2 add2(float2 a, float2 b) {
+  unsigned long long ra, rb, rc;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(ra) : "f"(a.x), "f"(a.y));
+  asm("mov.b64 %0, {%1, %2};" : "=l"(rb) : "f"(b.x), "f"(b.y));
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(rc) : "l"(ra), "l"(rb));
+  float2 c;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(c.x), "=f"(c.y) : "l"(rc));
+  return c;
+}
+__device__ __forceinline__ float2 mul2(float2 a, float2 b) {
+  unsigned long long ra, rb, rc;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(ra) : "f"(a.x), "f"(a.y));
+  asm("mov.b64 %0, {%1, %2};" : "=l"(rb) : "f"(b.x), "f"(b.y));
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(rc) : "l"(ra), "l"(rb));
+  float2 c;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(c.x), "=f"(c.y) : "l"(rc));
+  return c;
+}
+
+// a b rounded, as a packed FMA onto -0. The assembler contracts a packed multiply and
+// a packed add that follows it into one FMA, the .rn of both notwithstanding (every
+// one of 13157 sampled differences to the two roundings was the fused result), so
+// where both roundings count the product is formed here; ``nz`` is neg_zero(), a
+// value it cannot know.
+__device__ __forceinline__ float2 mul2_rn(float2 a, float2 b, float2 nz) {
+  unsigned long long ra, rb, rz, rc;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(ra) : "f"(a.x), "f"(a.y));
+  asm("mov.b64 %0, {%1, %2};" : "=l"(rb) : "f"(b.x), "f"(b.y));
+  asm("mov.b64 %0, {%1, %2};" : "=l"(rz) : "f"(nz.x), "f"(nz.y));
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(rc) : "l"(ra), "l"(rb), "l"(rz));
+  float2 c;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(c.x), "=f"(c.y) : "l"(rc));
+  return c;
+}
+// (the launches here are one-dimensional)
+__device__ __forceinline__ float2 neg_zero() {
+  const float z = __uint_as_float(0x80000000u ^ (gridDim.y - 1u));
+  return make_float2(z, z);
+}
+
+// A compile-time index as an argument.
+template <int V>
+struct IntTag {
+  static constexpr int value = V;
+};
+
 }  // namespace lrd

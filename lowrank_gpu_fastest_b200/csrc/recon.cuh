@@ -209,21 +209,46 @@ __device__ __forceinline__ void recon_body(const float* __restrict__ xc, const f
       const float4* vr = reinterpret_cast<const float4*>(vb + (size_t)kk * TP + t0);
       constexpr int CH = 4 / SPLIT;         // chunks per thread
       constexpr int CU4 = TPT / 4 / CH;     // float4 groups per chunk
+      // For the frame counts that have a warp kernel (chunks of 8, 12, 16 and 24
+      // frames) a chunk's even and odd frames are summed apart, as it does, and at T =
+      // 96 in two halves, which it gives to two lanes; other chunks in one sum.
+      constexpr bool EO = CU4 == 2 || CU4 == 3 || CU4 == 4 || CU4 == 6;
       float cp[CH];
+      auto sum_even_odd = [&](int c, auto from, auto to) {  // frame quads [from, to) of chunk c
+        float ev = 0.f, od = 0.f;
 #pragma unroll
-      for (int c = 0; c < CH; ++c) {
-        float acc_c = 0.f;
-#pragma unroll
-        for (int u4 = c * CU4; u4 < (c + 1) * CU4; ++u4) {
+        for (int i = decltype(from)::value; i < decltype(to)::value; ++i) {
+          const int u4 = c * CU4 + i;
           if (t0 + 4 * u4 < TP) {
             const float4 q = vr[u4];
-            acc_c = fmaf(xr[4 * u4 + 0], q.x, acc_c);
-            acc_c = fmaf(xr[4 * u4 + 1], q.y, acc_c);
-            acc_c = fmaf(xr[4 * u4 + 2], q.z, acc_c);
-            acc_c = fmaf(xr[4 * u4 + 3], q.w, acc_c);
+            ev = fmaf(xr[4 * u4 + 0], q.x, ev);
+            od = fmaf(xr[4 * u4 + 1], q.y, od);
+            ev = fmaf(xr[4 * u4 + 2], q.z, ev);
+            od = fmaf(xr[4 * u4 + 3], q.w, od);
           }
         }
-        cp[c] = acc_c;
+        return __fadd_rn(ev, od);
+      };
+#pragma unroll
+      for (int c = 0; c < CH; ++c) {
+        if (CU4 == 6 && T == 96) {
+          cp[c] = __fadd_rn(sum_even_odd(c, IntTag<0>{}, IntTag<3>{}), sum_even_odd(c, IntTag<3>{}, IntTag<6>{}));
+        } else if (EO) {
+          cp[c] = sum_even_odd(c, IntTag<0>{}, IntTag<CU4>{});
+        } else {
+          float acc_c = 0.f;
+#pragma unroll
+          for (int u4 = c * CU4; u4 < (c + 1) * CU4; ++u4) {
+            if (t0 + 4 * u4 < TP) {
+              const float4 q = vr[u4];
+              acc_c = fmaf(xr[4 * u4 + 0], q.x, acc_c);
+              acc_c = fmaf(xr[4 * u4 + 1], q.y, acc_c);
+              acc_c = fmaf(xr[4 * u4 + 2], q.z, acc_c);
+              acc_c = fmaf(xr[4 * u4 + 3], q.w, acc_c);
+            }
+          }
+          cp[c] = acc_c;
+        }
       }
       float part;
       if (CH == 4)
