@@ -101,9 +101,9 @@ __global__ void __launch_bounds__(32, eigh_reg_min_blocks<TMAX>()) eigh_reg_batc
 }
 
 template <int TMAX>
-__global__ void __launch_bounds__(TMAX) eigh_cta_batch_kernel(const BatchVol* __restrict__ vols,
-                                                              const int* __restrict__ list,
-                                                              const long long* __restrict__ off, int n) {
+__global__ void __launch_bounds__(TMAX, eigh_cta_min_blocks<TMAX>())
+    eigh_cta_batch_kernel(const BatchVol* __restrict__ vols, const int* __restrict__ list,
+                          const long long* __restrict__ off, int n) {
   const int i = batch_find(off, n, blockIdx.x);
   const BatchVol& V = vols[list[i]];
   eigh_cta_body<TMAX>(V.gv, V.gv, nullptr, V.rank, V.wgt, V.sig2, V.g.nt, V.g.nvox_patch, 0, V.refine,

@@ -387,12 +387,11 @@ __device__ __forceinline__ double mp_rank_sub(const float* lam, float unscale, i
 }
 
 // Eigenvectors of the tridiagonal for the eigenvalues lam[n - 1 - j0 - q], q < g <=
-// kInvGroup, unnormalised, entry i at Z[i * kInvGroup + q]. Two lanes per vector;
-// Z and U: TMAX x kInvGroup each.
-template <int TMAX>
+// kInvGroup, unnormalised, entry i at Z[i * kInvGroup + q], by the L lanes of a
+// matrix, two per vector. Z and U: n x kInvGroup each.
+template <int L>
 __device__ __forceinline__ void twisted_vectors(const float* d, const float* e, const float* lam, float* Z, float* U,
                                                 int n, int j0, int g, float tnorm) {
-  constexpr int L = eigh_reg_lanes<TMAX>();
   const int l = threadIdx.x & (L - 1);
   const int q = l & (kInvGroup - 1), down = (l / kInvGroup) & 1;  // down 0: from the top, 1: from the bottom
   const bool on = l < 2 * kInvGroup && q < g;
@@ -467,6 +466,72 @@ __device__ __forceinline__ void twisted_vectors(const float* d, const float* e, 
     }
   }
   __syncwarp();
+}
+
+// Modified Gram-Schmidt in descending eigenvalue order of the chunk's g vectors
+// (y[ri][q / 2] = vectors q, q + 1, row l + L ri), against each other and the j0
+// vectors before them, which are read from the output ``V``; then written there.
+// gmax >= g: vectors of the fullest matrix of the warp (one with fewer works on
+// zeros).
+template <int L, int R>
+__device__ __forceinline__ void gram_schmidt(float2 (&y)[R][kInvGroup / 2], float* V, int n, int j0, int g, int gmax,
+                                             bool mine) {
+  const int l = threadIdx.x & (L - 1);
+  auto vq = [&](int ri, int q) -> float& { return (q & 1) ? y[ri][q / 2].y : y[ri][q / 2].x; };
+#pragma unroll
+  for (int q = 0; q < kInvGroup; ++q) {
+    if (q >= gmax) continue;
+    auto norm2 = [&]() {
+      float s_ = 0.f;
+#pragma unroll
+      for (int ri = 0; ri < R; ++ri) s_ = fmaf(vq(ri, q), vq(ri, q), s_);
+      return sub_sum<L>(s_);
+    };
+    auto project = [&](const float (&w)[R], bool on) {  // takes the part along w out
+      float s_ = 0.f;
+#pragma unroll
+      for (int ri = 0; ri < R; ++ri) s_ = fmaf(w[ri], vq(ri, q), s_);
+      const float sum = sub_sum<L>(s_), dot = on ? sum : 0.f;  // (the shuffles by the whole warp)
+#pragma unroll
+      for (int ri = 0; ri < R; ++ri) vq(ri, q) = fmaf(-dot, w[ri], vq(ri, q));
+    };
+    const float before = norm2();
+    bool on = true;  // this matrix takes part
+#pragma unroll 1
+    for (int round = 0; round < 2; ++round) {
+      for (int i = 0; i < j0; ++i) {  // earlier chunks, from the output
+        float w[R];
+#pragma unroll
+        for (int ri = 0; ri < R; ++ri) w[ri] = (l + L * ri < n && q < g) ? V[(long long)i * n + l + L * ri] : 0.f;
+        project(w, on);
+      }
+#pragma unroll
+      for (int i = 0; i < q; ++i) {
+        float w[R];
+#pragma unroll
+        for (int ri = 0; ri < R; ++ri) w[ri] = vq(ri, i);
+        project(w, on);
+      }
+      const float after = norm2();
+      const float inv = on ? rsqrtf(fmaxf(after, FLT_MIN)) : 1.f;
+#pragma unroll
+      for (int ri = 0; ri < R; ++ri) vq(ri, q) *= inv;
+      // little left of it (nearly parallel to the earlier ones): once more, from
+      // the normalised rest
+      on = after < 1e-3f * before;
+      if (!__any_sync(0xffffffffu, on)) break;
+    }
+  }
+  if (mine) {
+#pragma unroll
+    for (int q = 0; q < kInvGroup; ++q)
+      if (q < g)
+#pragma unroll
+        for (int ri = 0; ri < R; ++ri) {
+          const int r = l + L * ri;
+          if (r < n) V[(long long)(j0 + q) * n + r] = vq(ri, q);
+        }
+  }
 }
 
 // Body of one warp's matrices ``b0``, b0 + 1 (the launch's patch index, below nmat;
@@ -711,7 +776,7 @@ __device__ __forceinline__ void eigh_reg_body(const float* gram, float* vecs, fl
   for (int j0 = 0; j0 < pmax; j0 += kInvGroup) {
     const int g = min(kInvGroup, p - j0);  // <= 0: this matrix has no more
     __syncwarp();
-    twisted_vectors<TMAX>(d, e, lam, Z, U, n, j0, g, tnorm);
+    twisted_vectors<L>(d, e, lam, Z, U, n, j0, g, tnorm);
     LRD_STAMP(5);
     // row-distributed: y[ri][q / 2] = vectors q, q + 1, row l + L ri
     float2 y[R][kInvGroup / 2];
@@ -761,64 +826,7 @@ __device__ __forceinline__ void eigh_reg_body(const float* gram, float* vecs, fl
     else
       back_transform(IntTag<4>{});
     LRD_STAMP(6);
-    // modified Gram-Schmidt in descending eigenvalue order (a matrix with fewer
-    // vectors than the other works on zeros)
-    auto vq = [&](int ri, int q) -> float& { return (q & 1) ? y[ri][q / 2].y : y[ri][q / 2].x; };
-    const int gmax = min(kInvGroup, pmax - j0);
-#pragma unroll
-    for (int q = 0; q < kInvGroup; ++q) {
-      if (q >= gmax) continue;
-      auto norm2 = [&]() {
-        float s_ = 0.f;
-#pragma unroll
-        for (int ri = 0; ri < R; ++ri) s_ = fmaf(vq(ri, q), vq(ri, q), s_);
-        return sub_sum<L>(s_);
-      };
-      auto project = [&](const float (&w)[R], bool on) {  // takes the part along w out
-        float s_ = 0.f;
-#pragma unroll
-        for (int ri = 0; ri < R; ++ri) s_ = fmaf(w[ri], vq(ri, q), s_);
-        const float dot = on ? sub_sum<L>(s_) : (sub_sum<L>(s_), 0.f);
-#pragma unroll
-        for (int ri = 0; ri < R; ++ri) vq(ri, q) = fmaf(-dot, w[ri], vq(ri, q));
-      };
-      const float before = norm2();
-      bool on = true;  // this matrix takes part
-#pragma unroll 1
-      for (int round = 0; round < 2; ++round) {
-        for (int i = 0; i < j0; ++i) {  // earlier chunks, from the output
-          float w[R];
-#pragma unroll
-          for (int ri = 0; ri < R; ++ri) w[ri] = (l + L * ri < n && q < g) ? V[(long long)i * n + l + L * ri] : 0.f;
-          project(w, on);
-        }
-#pragma unroll
-        for (int i = 0; i < q; ++i) {
-          float w[R];
-#pragma unroll
-          for (int ri = 0; ri < R; ++ri) w[ri] = vq(ri, i);
-          project(w, on);
-        }
-        const float after = norm2();
-        const float inv = on ? rsqrtf(fmaxf(after, FLT_MIN)) : 1.f;
-#pragma unroll
-        for (int ri = 0; ri < R; ++ri) vq(ri, q) *= inv;
-        // little left of it (nearly parallel to the earlier ones): once more, from
-        // the normalised rest
-        on = after < 1e-3f * before;
-        if (!__any_sync(0xffffffffu, on)) break;
-      }
-    }
-    if (mine) {
-#pragma unroll
-      for (int q = 0; q < kInvGroup; ++q)
-        if (q < g)
-#pragma unroll
-          for (int ri = 0; ri < R; ++ri) {
-            const int r = l + L * ri;
-            if (r < n) V[(long long)(j0 + q) * n + r] = vq(ri, q);
-          }
-    }
+    gram_schmidt<L, R>(y, V, n, j0, g, min(kInvGroup, pmax - j0), mine);
     __syncwarp();
   }
   LRD_STAMP(7);
