@@ -228,8 +228,9 @@ int lrd_denoise_static(const lrd_problem* problem, const float* d_vol, float* d_
  * per solver class T <= 32 / 48 / 64 / 96 / 128; near-tie pass: all;
  * reconstruction: per frame count and form), each block finding its volume
  * in a device table of per-volume descriptors. Volumes whose Gram or
- * reconstruction runs on another kernel (T % 4 != 0, the tcgen05 Gram of the
- * tensor form, an explicit brick) get per-volume launches in that phase.
+ * reconstruction runs on another kernel (the tcgen05 Gram of the tensor form, a
+ * frame count without a warp reconstruction, an explicit brick) get per-volume
+ * launches in that phase.
  * Every volume's result is bit-identical to lrd_denoise's. ``n_streams`` is
  * accepted for compatibility and unused: the launches run in order on
  * ``stream``.

@@ -73,12 +73,12 @@ __global__ void center_batch_kernel(const BatchVol* __restrict__ vols, const int
   const int i = batch_find(off, n, blockIdx.x);
   const BatchVol& V = vols[list[i]];
   const long long nvox = (long long)V.g.nx * V.g.ny * V.g.nz;
-  center_body(V.vol, V.xc, V.mean, nvox, V.g.nt, (long long)blockIdx.x - off[i]);
+  center_body(V.vol, V.xc, V.mean, nvox, V.g.nt, V.g.ldx, (long long)blockIdx.x - off[i]);
 }
 
 // Column Gram, every column of each listed volume (no short-last-wave cut: the
 // batch's columns fill the device; only a ring that does not fit is cut).
-template <int KS>
+template <int KS, bool EXACT>
 __global__ void __launch_bounds__(kGramzMaxThreads) gram_z_batch_kernel(const BatchVol* __restrict__ vols, const int* __restrict__ list,
                                                     const long long* __restrict__ off, int n) {
   const int i = batch_find(off, n, blockIdx.x);
@@ -86,7 +86,7 @@ __global__ void __launch_bounds__(kGramzMaxThreads) gram_z_batch_kernel(const Ba
   if (threadIdx.x == 0)  // the map was written by a copy before this launch; order it for the TMA unit
     asm volatile("fence.proxy.tensormap::generic.acquire.gpu [%0], 128;\n" ::"l"(&V.map) : "memory");
   const long long ncols = (long long)V.g.ncx * V.g.ncy;
-  gram_z_body<KS>(&V.map, V.gv, V.g, V.tab, 0, V.ring, V.cut > 1 ? 0 : (int)ncols, V.cut, V.status,
+  gram_z_body<KS, EXACT>(&V.map, V.gv, V.g, V.tab, 0, V.ring, V.cut > 1 ? 0 : (int)ncols, V.cut, V.status,
                   (int)(blockIdx.x - off[i]));
 }
 

@@ -503,6 +503,7 @@ __device__ __forceinline__ void eigh_refine_body(const float* __restrict__ vol, 
   const int nchunk = (nvox + rows - 1) / rows;
   const int ks = max(1, NT / nblk);  // threads per 4 x 4 block, splitting the rows
   const float* src = vol != nullptr ? vol : xc;
+  const int lds = vol != nullptr ? n : g.ldx;
   const double rn = vol != nullptr ? 1.0 / n : 0.0;  // 0: rows used as they are
   double* A = sm_ref;
   double* stage = sm_ref + refine_stage_at(n);
@@ -518,7 +519,7 @@ __device__ __forceinline__ void eigh_refine_body(const float* __restrict__ vol, 
       const int v = c * rows + sr;
       const bool ok = sr < rows && v < nvox;
       const int x = v / (g.py * g.pz), yz = v - x * (g.py * g.pz), y = yz / g.pz;
-      const float* p = src + (ok ? voxel_row(g, cx + x, cy + y, cz + (yz - y * g.pz)) * n : 0);
+      const float* p = src + (ok ? voxel_row(g, cx + x, cy + y, cz + (yz - y * g.pz)) * lds : 0);
 #pragma unroll
       for (int t = 0; t < 16; ++t)
         if (8 * t < n) pre[t] = (ok && l8 + 8 * t < n) ? p[l8 + 8 * t] : 0.f;

@@ -56,7 +56,7 @@ __global__ void gram_kernel(const float* __restrict__ xc, float* __restrict__ gr
     __syncthreads();
     // stage plane x = cx + a: rows (yy, zz) -> smem row yy*pz + zz, padded to ld
     for (int yy = 0; yy < g.py; ++yy) {
-      const float* src = xc + voxel_row(g, cx + a, cy + yy, cz) * T;
+      const float* src = xc + voxel_row(g, cx + a, cy + yy, cz) * T;  // (this kernel's volume is not padded)
       float* dst = plane + (size_t)yy * g.pz * ld;
       if (ld == T) {
         for (int e = tid; e < runlen; e += blockDim.x) dst[e] = src[e];

@@ -30,6 +30,11 @@
 // halving exchanges and added to the windows in float32, and a window is written
 // out (and its slot cleared) after its last plane. The K = px*py*pz sum therefore
 // rounds as a blocked sum: rows of a plane group, lanes, window.
+// A frame count that is not a multiple of 4 has the rows of its centred volume padded
+// to one with zeros (TMA strides are multiples of 16 bytes), and its windows add
+// without rounding (gramz_exact): with a CTA per patch 61x53x37x65 / 7^3 / stride 2
+// 1.49 ms, 0.61 here (0.39 with windows rounded at each plane, but 4% further from
+// the float64 Gram at T = 17 and 31); 40x40x32x127 2.15 and 0.71.
 // Tried and dropped (headline ms): a producer warp with chunks of x-rows and no
 // CTA barrier 0.59 (its warp leaves one of the SM's four schedulers idle), the
 // same with thread 0 of the first warp as producer 0.63, the next row's loads
@@ -103,27 +108,54 @@ __host__ __device__ inline size_t gramz_plane_floats(int rows, int T) {
 
 // 8 x 8 blocks of the upper block triangle: block b of nb = ceil(T / 8) owns the
 // 4-frame quads b and b + nb (the second one absent at the end of an odd count).
-__host__ __device__ inline int gramz_nb(int T) { return ((T >> 2) + 1) >> 1; }
+__host__ __device__ inline int gramz_nb(int T) { return (((T + 3) >> 2) + 1) >> 1; }
 __host__ __device__ inline int gramz_nblk(int T) {
   const int nb = gramz_nb(T);
   return nb * (nb + 1) / 2;
 }
 
-// Threads of a column CTA for T frames and K-split ks: the blocks, 32 / ks to a
+// Whether the windows add their planes without rounding (a high and a low word): the
+// frame counts that are not a multiple of 4, which a CTA per patch summed over planes
+// in float64 before their rows were padded for this kernel.
+__host__ __device__ inline bool gramz_exact(int T) { return (T & 3) != 0; }
+
+// CTAs that share a column's blocks: two for the 136 blocks of T > 120, which four
+// lanes each would make 17 warps of 128 registers (two lanes each sum 61 rows of an
+// 11 x 11 plane one after the other: 11^3 / stride 2 / T = 128 6.2e-8 of the Gram
+// off against 5.5e-8).
+__host__ __device__ inline int gramz_shares(int T, int ks) { return ks >= 4 && gramz_nblk(T) > 128 ? 2 : 1; }
+__host__ __device__ inline int gramz_cta_blocks(int T, int ks) {
+  return gramz_nblk(T) / gramz_shares(T, ks);  // (136 or a share of one)
+}
+
+// Threads of a column CTA for T frames and K-split ks: its blocks, 32 / ks to a
 // warp, times ks.
 __host__ __device__ inline int gramz_threads(int T, int ks) {
   const int per_warp = 32 / ks;
-  return 32 * ((gramz_nblk(T) + per_warp - 1) / per_warp);
+  return 32 * ((gramz_cta_blocks(T, ks) + per_warp - 1) / per_warp);
 }
 
 // Dynamic shared memory: two plane slots, ``ring`` window accumulators (64 floats
-// per block), two mbarriers.
-__host__ __device__ inline size_t gramz_smem_bytes(int px, int py, int T, int ring) {
-  return sizeof(float) * (2 * gramz_plane_floats(px * py, T) + (size_t)ring * 64 * gramz_nblk(T)) + 2 * sizeof(uint64_t);
+// per block, twice that where they carry their rounding errors), two mbarriers.
+__host__ __device__ inline size_t gramz_smem_bytes(int px, int py, int T, int ks, int ring) {
+  return sizeof(float) * (2 * gramz_plane_floats(px * py, (T + 3) & ~3) +
+                          (size_t)ring * (gramz_exact(T) ? 128 : 64) * gramz_cta_blocks(T, ks)) +
+         2 * sizeof(uint64_t);
 }
 
-// grid: nfull + (columns - nfull) * nsplit CTAs; block: gramz_threads(T, KS)
-// (T % 4 == 0, KS in {2, 4, 8}). CTA b < nfull computes every window of column
+// (hi, lo) += x: Knuth's two-sum, its error into lo.
+__device__ __forceinline__ void add_exact(float& hi, float& lo, float x) {
+  const float s = __fadd_rn(hi, x), b = __fsub_rn(s, hi);
+  lo = __fadd_rn(lo, __fadd_rn(__fsub_rn(hi, __fsub_rn(s, b)), __fsub_rn(x, b)));
+  hi = s;
+}
+
+// (an overflowed sum's error term is a NaN)
+__device__ __forceinline__ float joined(float hi, float lo) { return lo == lo ? __fadd_rn(hi, lo) : hi; }
+
+// grid: gramz_shares(T, KS) CTAs, neighbours, for each of nfull + (columns - nfull) *
+// nsplit units; block: gramz_threads(T, KS)
+// (KS in {2, 4, 8}; voxel rows of ldx = 4 ceil(T / 4) floats). Unit b < nfull computes every window of column
 // col0 + b; the columns after the first nfull are each cut into nsplit units
 // of consecutive windows (a unit reads only the planes of its windows; it needs
 // min(windows active at a plane, windows of the unit) <= ring), so a launch
@@ -133,25 +165,29 @@ __host__ __device__ inline size_t gramz_smem_bytes(int px, int py, int T, int ri
 // does not depend on the cut. ``col0`` = first column (x-major index
 // ci * ncy + cj); ``gram`` points at the Gram block of the launch's first
 // patch (patch index col0 * ncz).
-// Body of one CTA (index ``bid``); ``xmap`` points at the tensor map (a kernel
+// Body of one CTA (index ``cta``); ``xmap`` points at the tensor map (a kernel
 // parameter, or a 64-byte aligned copy in global memory for the packed
 // multi-volume launch).
-template <int KS>
+template <int KS, bool EXACT>
 __device__ __forceinline__ void gram_z_body(const CUtensorMap* xmap, float* __restrict__ gram, const Geom& g,
                                             const AxisTables& tab, long long col0, int ring, int nfull, int nsplit,
-                                            int* status, int bid) {
+                                            int* status, int cta) {
   static_assert(KS == 2 || KS == 4 || KS == 8, "threads per block");
   constexpr int BW = 32 / KS;  // blocks per warp: lane = kq * BW + block
   constexpr int NR = 8 / KS;   // rows of its block a thread ends up with: kq * NR ...
   extern __shared__ __align__(128) float smz[];
-  const int T = g.nt;
+  const int T = g.nt, ldx = EXACT ? (T + 3) & ~3 : T;  // (g.ldx)
   const int rows = g.px * g.py;
-  const size_t pf = gramz_plane_floats(rows, T);
-  const int nq = T >> 2, nb = gramz_nb(T), nblk = gramz_nblk(T);
+  const size_t pf = gramz_plane_floats(rows, ldx);
+  const int nq = ldx >> 2, nb = gramz_nb(T);
+  // this CTA's blocks (of two, 68 each)
+  const int shares = gramz_shares(T, KS), nblk = gramz_nblk(T) / shares;
+  const int bid = shares == 2 ? cta >> 1 : cta, blk0 = shares == 2 ? (cta & 1) * nblk : 0;
   const int nthreads = blockDim.x;
   const int nown = nblk * KS;                             // threads that own a share of a block
-  float4* win = reinterpret_cast<float4*>(smz + 2 * pf);  // [ring][2 NR][nown]
-  uint64_t* bars = reinterpret_cast<uint64_t*>(smz + 2 * pf + (size_t)ring * 64 * nblk);
+  constexpr int SLOT = EXACT ? 32 : 16;  // float4s of a window per block
+  float4* win = reinterpret_cast<float4*>(smz + 2 * pf);  // [ring][high(, low)][2 NR][nown]
+  uint64_t* bars = reinterpret_cast<uint64_t*>(win + (size_t)ring * SLOT * nblk);
   const uint32_t bar0 = (uint32_t)__cvta_generic_to_shared(bars);
 
   // this CTA's column and windows [wlo, whi]
@@ -167,7 +203,7 @@ __device__ __forceinline__ void gram_z_body(const CUtensorMap* xmap, float* __re
   const bool owner = blk < nblk;
   int bi = 0, bj = 0;
   if (owner) {
-    int rem = blk;
+    int rem = blk0 + blk;
     while (rem >= nb - bi) {
       rem -= nb - bi;
       ++bi;
@@ -177,13 +213,13 @@ __device__ __forceinline__ void gram_z_body(const CUtensorMap* xmap, float* __re
   // quads of the block's rows and columns (an absent one reads the last quad;
   // what comes of it is not stored)
   const int qa0 = bi, qa1 = min(bi + nb, nq - 1), qb0 = bj, qb1 = min(bj + nb, nq - 1);
-  const uint32_t plane_bytes = (uint32_t)(rows * T * sizeof(float));
+  const uint32_t plane_bytes = (uint32_t)(rows * ldx * sizeof(float));
   auto fetch = [&](int z, int slot) {  // plane z into a slot that nothing reads or fills
     mbar_expect_tx(bar0 + 8 * slot, plane_bytes);
     tma_load_4d((uint32_t)__cvta_generic_to_shared(smz + slot * pf), xmap, bar0 + 8 * slot, 0, z, cy, cx);
   };
 
-  for (int e = tid; e < ring * 16 * nblk; e += nthreads) win[e] = make_float4(0.f, 0.f, 0.f, 0.f);
+  for (int e = tid; e < ring * SLOT * nblk; e += nthreads) win[e] = make_float4(0.f, 0.f, 0.f, 0.f);
   if (tid == 0) {
     mbar_init(bar0, 1);
     mbar_init(bar0 + 8, 1);
@@ -192,7 +228,8 @@ __device__ __forceinline__ void gram_z_body(const CUtensorMap* xmap, float* __re
   __syncthreads();
   if (tid == 0 && zlo <= zhi) fetch(zlo, 0);
   float* G0 = gram + (size_t)((col - col0) * g.ncz) * T * T;
-  const bool aligned = (reinterpret_cast<uintptr_t>(gram) & 15) == 0;  // a caller's block may not be
+  // rows of G take float4 (a caller's block may not be aligned)
+  const bool aligned = !EXACT && (reinterpret_cast<uintptr_t>(gram) & 15) == 0;
   float2 acc[8][4];  // row u of the block, column pairs
 #pragma unroll
   for (int u = 0; u < 8; ++u)
@@ -304,7 +341,7 @@ __device__ __forceinline__ void gram_z_body(const CUtensorMap* xmap, float* __re
     const bool klo_ends = z == tab.corners[2][klo] + g.pz - 1;
     int wslot = klo % ring;
     for (int k = klo; k <= khi; ++k) {
-      float4* w = win + (size_t)wslot * 16 * nblk + kq * nblk + blk;
+      float4* w = win + (size_t)wslot * SLOT * nblk + kq * nblk + blk;
       const bool ends = k == klo && klo_ends;
       float* G = G0 + (size_t)k * T * T;
 #pragma unroll
@@ -312,11 +349,23 @@ __device__ __forceinline__ void gram_z_body(const CUtensorMap* xmap, float* __re
 #pragma unroll
         for (int cq = 0; cq < 2; ++cq) {  // the row's two column quads
           float4 v = w[(2 * u + cq) * nown];
-          v.x += mine[u][2 * cq].x;
-          v.y += mine[u][2 * cq].y;
-          v.z += mine[u][2 * cq + 1].x;
-          v.w += mine[u][2 * cq + 1].y;
-          w[(2 * u + cq) * nown] = ends ? make_float4(0.f, 0.f, 0.f, 0.f) : v;
+          if constexpr (EXACT) {
+            float4& low = w[(2 * (NR + u) + cq) * nown];
+            float4 l = low;
+            add_exact(v.x, l.x, mine[u][2 * cq].x);
+            add_exact(v.y, l.y, mine[u][2 * cq].y);
+            add_exact(v.z, l.z, mine[u][2 * cq + 1].x);
+            add_exact(v.w, l.w, mine[u][2 * cq + 1].y);
+            low = ends ? make_float4(0.f, 0.f, 0.f, 0.f) : l;
+            w[(2 * u + cq) * nown] = ends ? make_float4(0.f, 0.f, 0.f, 0.f) : v;
+            v = make_float4(joined(v.x, l.x), joined(v.y, l.y), joined(v.z, l.z), joined(v.w, l.w));
+          } else {
+            v.x += mine[u][2 * cq].x;
+            v.y += mine[u][2 * cq].y;
+            v.z += mine[u][2 * cq + 1].x;
+            v.w += mine[u][2 * cq + 1].y;
+            w[(2 * u + cq) * nown] = ends ? make_float4(0.f, 0.f, 0.f, 0.f) : v;
+          }
           const int ub = kq * NR + u;  // row of the block
           const int fr = ub < 4 ? 4 * bi + ub : 4 * (bi + nb) + ub - 4, qc = cq ? bj + nb : bj;
           if (ends && fr < T && qc < nq) {
@@ -324,17 +373,17 @@ __device__ __forceinline__ void gram_z_body(const CUtensorMap* xmap, float* __re
             if (aligned) {
               *reinterpret_cast<float4*>(gr) = v;
             } else {
-              gr[0] = v.x;
-              gr[1] = v.y;
-              gr[2] = v.z;
-              gr[3] = v.w;
+              const float vs[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+              for (int i = 0; i < 4; ++i)
+                if (!EXACT || 4 * qc + i < T) gr[i] = vs[i];
             }
             if (bi != bj) {
               float* gc = G + (size_t)(4 * qc) * T + fr;
-              gc[0] = v.x;
-              gc[T] = v.y;
-              gc[2 * (size_t)T] = v.z;
-              gc[3 * (size_t)T] = v.w;
+              const float vs[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+              for (int i = 0; i < 4; ++i)
+                if (!EXACT || 4 * qc + i < T) gc[i * (size_t)T] = vs[i];
             }
           }
         }
@@ -343,14 +392,14 @@ __device__ __forceinline__ void gram_z_body(const CUtensorMap* xmap, float* __re
   }
 }
 
-// (T <= 128 needs at most 544 threads at KS = 4, 288 at KS = 2; KS = 8 runs up to T = 88)
+// (KS = 4 needs at most 480 threads, KS = 2 288; KS = 8 runs up to T = 80)
 constexpr int kGramzMaxThreads = 512;
 
-template <int KS>
+template <int KS, bool EXACT>
 __global__ void __maxnreg__(128)
     gram_z_kernel(const __grid_constant__ CUtensorMap xmap, float* __restrict__ gram, Geom g, AxisTables tab,
                   long long col0, int ring, int nfull, int nsplit, int* status) {
-  gram_z_body<KS>(&xmap, gram, g, tab, col0, ring, nfull, nsplit, status, (int)blockIdx.x);
+  gram_z_body<KS, EXACT>(&xmap, gram, g, tab, col0, ring, nfull, nsplit, status, (int)blockIdx.x);
 }
 
 // Self-test of the bounded wait: one thread waits on a freshly initialised

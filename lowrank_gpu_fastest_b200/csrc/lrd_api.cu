@@ -88,11 +88,10 @@ struct lrd_plan {
   int gramz_ks = 4;        // voxel-row split per 8x8 Gram block (threads per block)
   bool eigh_cta = false;   // eigensolver: one CTA per matrix (else one warp)
   size_t smem_gramz;
-  int gramz_slots = 0;     // column CTAs resident at once on the device (0: never cut columns)
+  int gramz_slots = 0;     // columns resident at once on the device (0: never cut columns)
   int gramtc_slots = 0;    // the same for the tensor-core column Gram
   int sms = 0;             // multiprocessors of the device
-  size_t smem_center, smem_gram, smem_eigh, smem_recon;
-  int center_warps;
+  size_t smem_gram, smem_eigh, smem_recon;
   // workspace offsets (bytes)
   size_t off_mean, off_xc, off_gv, off_rank, off_wgt, off_sig2, off_status, off_refine, ws_bytes;
   size_t smem_refine;
@@ -147,19 +146,21 @@ namespace {
 // 0.52 (48x48x24x48 0.125 / 0.097 / 0.090: 8 there); 96x96x48x32, 5^3, stride 1
 // 1.77 / 1.40 / 1.69; 101x87x43x64, 7^3, stride 2 1.17 / 0.98 / 1.50;
 // 64x64x48x96, 11^3, stride 3 0.90 / 0.70 / -. A CTA of fewer than 48 threads at
-// 4 (T <= 24) takes 8. The split does not depend on the launch: it changes the
+// 4 (T <= 24) takes 8. Frame counts not a multiple of 4 take 4: 48x48x40 / 7^3 / stride
+// 2 at T = 17, 31, 53, 65, 127 0.15 / 0.09 / 0.10, 0.23 / 0.15 / 0.15, 0.45 / 0.29 /
+// 0.31, 0.73 / 0.48 / 0.50, 1.94 / 1.40 / -. The split does not depend on the launch: it changes the
 // rounding.
-int gramz_split(int T) { return (T <= 24 || (T > 40 && T <= 56)) ? 8 : 4; }
+int gramz_split(int T) { return !lrd::gramz_exact(T) && (T <= 24 || (T > 40 && T <= 56)) ? 8 : 4; }
 
 void* gramtc_kernel_ptr(bool bf16) {
   return bf16 ? (void*)lrd::gram_tc_kernel<true> : (void*)lrd::gram_tc_kernel<false>;
 }
 
-void* gramz_kernel_ptr(int ks) {
+void* gramz_kernel_ptr(int ks, bool exact) {
   switch (ks) {
-    case 2: return (void*)lrd::gram_z_kernel<2>;
-    case 8: return (void*)lrd::gram_z_kernel<8>;
-    default: return (void*)lrd::gram_z_kernel<4>;
+    case 2: return exact ? (void*)lrd::gram_z_kernel<2, true> : (void*)lrd::gram_z_kernel<2, false>;
+    case 8: return exact ? (void*)lrd::gram_z_kernel<8, true> : (void*)lrd::gram_z_kernel<8, false>;
+    default: return exact ? (void*)lrd::gram_z_kernel<4, true> : (void*)lrd::gram_z_kernel<4, false>;
   }
 }
 
@@ -368,11 +369,11 @@ int run_center(const lrd_plan* P, const float* d_vol, char* ws, cudaStream_t st,
   if (nv <= 0) return LRD_OK;
   float* mean = reinterpret_cast<float*>(ws + P->off_mean);
   float* xc = reinterpret_cast<float*>(ws + P->off_xc);
-  const int T = P->g.nt;
-  const long long per_block = 32LL * P->center_warps;
+  const int T = P->g.nt, ldx = P->g.ldx;
+  const long long per_block = lrd::center_block_rows();
   const long long blocks = (nv + per_block - 1) / per_block;
-  lrd::center_kernel<<<(unsigned)blocks, 32 * P->center_warps, P->smem_center, st>>>(
-      d_vol + v0 * T, xc + v0 * T, mean + v0, nv, T);
+  lrd::center_kernel<<<(unsigned)blocks, 32 * lrd::kCenterWarps, 0, st>>>(
+      d_vol + v0 * T, xc + v0 * ldx, mean + v0, nv, T, ldx);
   return launch_check("center_kernel launch");
 }
 
@@ -396,10 +397,10 @@ int encode_plane_map(const lrd_plan* P, const float* xc, CUtensorMap* map) {
   auto enc = tensor_map_encoder();
   if (!enc) return fail(LRD_ERR_CUDA, "cuTensorMapEncodeTiled is not available from the driver");
   const lrd::Geom& g = P->g;
-  const cuuint64_t dims[4] = {(cuuint64_t)g.nt, (cuuint64_t)g.nz, (cuuint64_t)g.ny, (cuuint64_t)g.nx};
-  const cuuint64_t strides[3] = {(cuuint64_t)g.nt * 4, (cuuint64_t)g.nz * g.nt * 4,
-                                 (cuuint64_t)g.ny * g.nz * g.nt * 4};
-  const cuuint32_t box[4] = {(cuuint32_t)g.nt, 1, (cuuint32_t)g.py, (cuuint32_t)g.px};
+  const cuuint64_t dims[4] = {(cuuint64_t)g.ldx, (cuuint64_t)g.nz, (cuuint64_t)g.ny, (cuuint64_t)g.nx};
+  const cuuint64_t strides[3] = {(cuuint64_t)g.ldx * 4, (cuuint64_t)g.nz * g.ldx * 4,
+                                 (cuuint64_t)g.ny * g.nz * g.ldx * 4};
+  const cuuint32_t box[4] = {(cuuint32_t)g.ldx, 1, (cuuint32_t)g.py, (cuuint32_t)g.px};
   const cuuint32_t estr[4] = {1, 1, 1, 1};
   CUresult r = enc(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, const_cast<float*>(xc), dims, strides, box, estr,
                    CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
@@ -454,15 +455,15 @@ int run_gram(const lrd_plan* P, char* ws, float* d_gram, cudaStream_t st, long l
               map, d_gram + c0 * P->g.ncz * TT, P->g, P->tab, c0, P->gramtc_ring, (int)nfull, nsplit, status);
         rc = launch_check("gram_tc_kernel launch");
       } else {
-        void* fn = gramz_kernel_ptr(P->gramz_ks);
+        void* fn = gramz_kernel_ptr(P->gramz_ks, lrd::gramz_exact(P->g.nt));
         float* gout = d_gram + c0 * P->g.ncz * TT;
         lrd::Geom gg = P->g;
         lrd::AxisTables tt = P->tab;
         int ring = P->gramz_ring, nf = (int)nfull;
         void* args[] = {(void*)&map, (void*)&gout, (void*)&gg, (void*)&tt, (void*)&c0, (void*)&ring,
                         (void*)&nf, (void*)&nsplit, (void*)&status};
-        cudaError_t le = cudaLaunchKernel(fn, dim3((unsigned)grid), dim3(lrd::gramz_threads(P->g.nt, P->gramz_ks)),
-                                          args, P->smem_gramz, st);
+        cudaError_t le = cudaLaunchKernel(fn, dim3((unsigned)(grid * lrd::gramz_shares(P->g.nt, P->gramz_ks))),
+                                          dim3(lrd::gramz_threads(P->g.nt, P->gramz_ks)), args, P->smem_gramz, st);
         if (le != cudaSuccess) return cuda_fail(le, "gram_z_kernel launch");
         rc = launch_check("gram_z_kernel launch");
       }
@@ -794,8 +795,6 @@ int create_plan(const lrd_problem* pr, const std::vector<int32_t>* x_corners, lr
   }
   const int nb4 = (T + 3) / 4;
   P->gram_threads = nb4 * (nb4 + 1) / 2;
-  P->center_warps = 4;
-  P->smem_center = sizeof(float) * (size_t)P->center_warps * (32 * (T + 1) + 32);
   P->smem_gram = sizeof(float) * (size_t)pr->py * pr->pz * (4 * nb4);
   P->eigh_cta = eigh_use_cta(T, pr->eigh_block);
   P->smem_eigh = sizeof(float) * eigh_smem_for(T, P->eigh_cta);
@@ -809,19 +808,21 @@ int create_plan(const lrd_problem* pr, const std::vector<int32_t>* x_corners, lr
     // The window ring, or the part of it that fits beside the planes (the
     // columns are then cut into ranges of that many windows).
     P->gramz_ring = ring;
-    while (P->gramz_ring > 1 && lrd::gramz_smem_bytes(pr->px, pr->py, T, P->gramz_ring) > kSmemMax) --P->gramz_ring;
+    while (P->gramz_ring > 1 && lrd::gramz_smem_bytes(pr->px, pr->py, T, P->gramz_ks, P->gramz_ring) > kSmemMax) --P->gramz_ring;
     P->gramz_cut = P->gramz_ring < ring ? (g.ncz + P->gramz_ring - 1) / P->gramz_ring : 1;
-    P->smem_gramz = lrd::gramz_smem_bytes(pr->px, pr->py, T, P->gramz_ring);
-    P->use_gramz = (T % 4 == 0) && P->smem_gramz <= kSmemMax && tensor_map_encoder() != nullptr &&
+    P->smem_gramz = lrd::gramz_smem_bytes(pr->px, pr->py, T, P->gramz_ks, P->gramz_ring);
+    // (a frame count that is not a multiple of 4 has its centred volume padded to
+    // one: TMA strides are multiples of 16 bytes)
+    P->use_gramz = P->smem_gramz <= kSmemMax && tensor_map_encoder() != nullptr &&
                    pr->px <= 256 && pr->py <= 256;
+    g.ldx = P->use_gramz ? (T + 3) & ~3 : T;
     P->gramtc_bf16 = pr->form == LRD_FORM_TENSOR_BF16;
     P->smem_gramtc = lrd::gramtc_smem_bytes(pr->px * pr->py, T, ring, P->gramtc_bf16);
     P->use_gramtc = (pr->form == LRD_FORM_TENSOR || pr->form == LRD_FORM_TENSOR_BF16) && T <= 64 && (T % 4 == 0) && pr->px * pr->py <= 128 &&
                     P->smem_gramtc <= 200 * 1024 && tensor_map_encoder() != nullptr;
   }
-  int rc = set_smem((const void*)lrd::center_kernel, P->smem_center);
-  if (!rc) rc = set_smem((const void*)lrd::gram_kernel, P->smem_gram);
-  if (!rc && P->use_gramz) rc = set_smem(gramz_kernel_ptr(P->gramz_ks), P->smem_gramz);
+  int rc = set_smem((const void*)lrd::gram_kernel, P->smem_gram);
+  if (!rc && P->use_gramz) rc = set_smem(gramz_kernel_ptr(P->gramz_ks, lrd::gramz_exact(T)), P->smem_gramz);
   if (!rc && P->use_gramtc) rc = set_smem(gramtc_kernel_ptr(P->gramtc_bf16), P->smem_gramtc);
   P->smem_refine = lrd::eigh_refine_smem_bytes(T);
   if (!rc) rc = set_smem((const void*)lrd::eigh_refine_kernel, P->smem_refine);
@@ -832,10 +833,10 @@ int create_plan(const lrd_problem* pr, const std::vector<int32_t>* x_corners, lr
     P->sms = sms;
     int per_sm = 0;
     if (!rc && P->use_gramz) {
-      if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, gramz_kernel_ptr(P->gramz_ks),
+      if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, gramz_kernel_ptr(P->gramz_ks, lrd::gramz_exact(T)),
                                                         lrd::gramz_threads(T, P->gramz_ks),
                                                         P->smem_gramz) == cudaSuccess)
-        P->gramz_slots = per_sm * sms;
+        P->gramz_slots = per_sm * sms / lrd::gramz_shares(T, P->gramz_ks);
       else
         (void)cudaGetLastError();  // no cut columns; the launches report their own errors
     }
@@ -922,7 +923,7 @@ int create_plan(const lrd_problem* pr, const std::vector<int32_t>* x_corners, lr
   // workspace layout
   size_t off = 0;
   P->off_mean = off; off += align256(sizeof(float) * (size_t)nvox);
-  P->off_xc = off; off += align256(sizeof(float) * (size_t)nvox * T);
+  P->off_xc = off; off += align256(sizeof(float) * (size_t)nvox * g.ldx);
   P->off_gv = off; off += align256(sizeof(float) * (size_t)g.npatch * T * T);
   P->off_rank = off; off += align256(sizeof(int32_t) * (size_t)g.npatch);
   P->off_wgt = off; off += align256(sizeof(float) * (size_t)g.npatch);

@@ -22,6 +22,7 @@ struct AxisTables {
 
 struct Geom {
   int nx, ny, nz, nt;      // volume
+  int ldx;                 // floats per voxel row of the centred volume: nt, or nt rounded up to 4 (zeros)
   int px, py, pz;          // patch
   int ncx, ncy, ncz;       // corners per axis
   long long npatch;        // ncx*ncy*ncz

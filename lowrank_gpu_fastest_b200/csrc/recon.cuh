@@ -140,7 +140,7 @@ __device__ __forceinline__ void recon_body(const float* __restrict__ xc, const f
 #pragma unroll
   for (int u = 0; u < TPT; ++u) {
     const int t = t0 + u;
-    xr[u] = (valid && t < T) ? xc[row * T + t] : 0.f;
+    xr[u] = (valid && t < T) ? xc[row * g.ldx + t] : 0.f;
     if constexpr (ACCURATE)
       acc64[u] = 0.0;
     else

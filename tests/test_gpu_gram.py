@@ -19,12 +19,15 @@ pytestmark = pytest.mark.gpu
 # quads of the 8 x 8 blocks even and odd in number (T % 8), one block (T = 4, 8),
 # row counts off the split (odd patches, one-voxel planes), a stride beyond the
 # patch (planes in no window), a border-shifted last corner, and window rings
-# that do not fit shared memory (T = 96 and 128 at stride 1: columns cut)
+# that do not fit shared memory (T = 96 and 128 at stride 1: columns cut); frame
+# counts whose rows are padded (T % 4)
 @pytest.mark.parametrize("shape,patch,stride,split", [
     ((7, 6, 9, 4), (3, 2, 3), 2, 0), ((9, 8, 7, 8), (3, 3, 3), 1, 4), ((8, 9, 13, 12), (5, 3, 4), 2, 1),
     ((9, 9, 12, 20), (1, 5, 5), 1, 0), ((9, 9, 12, 20), (5, 1, 5), 3, 2), ((12, 11, 17, 44), (5, 5, 5), 7, 0),
     ((12, 12, 14, 48), (5, 6, 5), 3, 4), ((12, 12, 16, 64), (5, 5, 5), 1, 0), ((13, 12, 15, 96), (11, 11, 11), 1, 0),
     ((8, 8, 12, 100), (5, 5, 5), 2, 0), ((8, 9, 14, 128), (7, 7, 7), 1, 4),
+    ((7, 6, 9, 2), (3, 2, 3), 2, 0), ((7, 6, 9, 5), (3, 3, 3), 1, 0), ((8, 9, 13, 31), (5, 4, 4), 2, 2),
+    ((9, 8, 11, 65), (5, 5, 5), 2, 0), ((13, 12, 15, 99), (11, 11, 11), 1, 0), ((8, 8, 9, 126), (6, 6, 5), 2, 1),
 ])
 def test_column_gram_vs_float64(cuda_ok, shape, patch, stride, split):
     rng = np.random.default_rng(shape[3])
