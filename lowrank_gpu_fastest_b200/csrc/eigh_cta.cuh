@@ -298,19 +298,14 @@ __device__ __forceinline__ void eigh_cta_body(const float* gram, float* vecs, fl
 
   // ---- MP rank (first warp) -------------------------------------------------------
   int* pshare = reinterpret_cast<int*>(scal + 1);
+  bool queue = false;  // (first warp; as in eigh_reg_body)
   if (warp == 0) {
     int p;
-    const double margin = mp_rank_sub<32>(lam, unscale, n, nvox, W, p, sig2 ? sig2 + b : nullptr);
+    queue = mp_rank_sub<32>(lam, unscale, n, nvox, W, p, sig2 ? sig2 + b : nullptr) < kRefineTol;
     if (lane == 0) {
       ranks[b] = p;
       wgt[b] = (float)(1.0 / (2.0 + (double)p));
       *pshare = p;
-      bool queue = margin < kRefineTol;  // (as in eigh_reg_body)
-      for (int j = 1; j < p; ++j) {
-        const float lo = lam[n - 1 - j], hi = lam[n - j];
-        queue |= hi - lo < 4.f * eps * tnorm && lo > 64.f * eps * tnorm;
-      }
-      if (refine_count != nullptr && queue) refine_ids[atomicAdd(refine_count, 1)] = (int)(patch0 + b);
     }
   }
   if (lam_out != nullptr && rv) lam_out[b * n + tid] = lam[tid] * unscale;
@@ -393,10 +388,11 @@ __device__ __forceinline__ void eigh_cta_body(const float* gram, float* vecs, fl
           z[ri][q / 2] = make_float2(r < n && q < g ? zz.x : 0.f, r < n && q + 1 < g ? zz.y : 0.f);
         }
       }
-      gram_schmidt<32, R>(z, V, n, j0, g, g, true);
+      queue |= gram_schmidt<32, R>(z, V, lam, tnorm, n, j0, g, g, true);
     }
     __syncthreads();
   }
+  if (tid == 0 && refine_count != nullptr && queue) refine_ids[atomicAdd(refine_count, 1)] = (int)(patch0 + b);
   LRD_STAMP(7);
 }
 

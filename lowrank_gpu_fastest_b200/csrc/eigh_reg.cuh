@@ -3,8 +3,8 @@
 // Householder tridiagonalisation, eigenvalues by Sturm counts, MP rank, the top-p
 // eigenvectors of the tridiagonal by twisted factorisations, back-transform,
 // Gram-Schmidt. L lanes hold one matrix in registers, rows l, l + L, ... of lane
-// l (every column index compile-time): L = 16 for TMAX <= 48, so a warp solves two
-// matrices side by side, L = 32 for TMAX = 64.
+// l (every column index compile-time): L = 8 for TMAX = 32, so a warp solves four
+// matrices side by side, L = 16 for 48 (two), L = 32 for 64.
 //
 // A reduction step is a chain of a dozen dependent stages (norm, reflector,
 // matrix-vector product, dot product, update), and only a quarter of its
@@ -32,18 +32,20 @@
 //
 // Measured on B200 (kernel time, against one matrix per warp with bisection by the
 // quotient recurrence and inverse iteration by partial-pivoting LU): 12600 matrices
-// at T = 48 0.885 -> 0.52 ms, 372416 at T = 32 11.5 -> 5.4, 37392 at T = 64 4.55 -> 2.9,
-// one matrix 105 -> 97 us. Cycles per warp at T = 48, 12 warps per SM (two matrices):
+// at T = 48 0.885 -> 0.52 ms, 372416 at T = 32 11.5 -> 5.2 (16 lanes per matrix 5.5),
+// 37392 at T = 64 4.55 -> 2.75, one matrix 105 -> 97 us. Cycles per warp at T = 48, 12 warps per SM (two matrices):
 // load 9 K, reduction 128 K, eigenvalues 67 K, rank 5 K, vectors 18 K, back-transform
 // 15 K, Gram-Schmidt 4 K (one matrix per warp at 16 warps: 12 / 147 / 93 / 6 / 29 / 22 /
 // 4 K). Instruction issue 46%, three warps per scheduler: latency bounds it, the
 // 168 registers of 12 warps and the shared memory bound the warps. Measured slower:
 // the reduction as four straight-line loops without the dead column groups of each
 // quarter (T = 48 alone 107 -> 71 K cycles, but 11 warps: 0.74 -> 0.77 ms; T = 64 3.10 ->
-// 3.39), points shared out among the intervals (12 rounds instead of 20, twice the
+// 3.39), the update as two rank-1 passes with the reflector read two groups ahead
+// (T = 48 0.75, T = 32 no change), points shared out among the intervals (12 rounds instead of 20, twice the
 // instructions around them: 0.80), two points per eigenvalue (0.83).
 //
-// The near-tie test (mp_rank's margin) queues patches for the float64 pass.
+// The near-tie test (mp_rank's margin) and vectors that coincide queue patches for the
+// float64 pass.
 #pragma once
 
 #include "eigh.cuh"
@@ -62,11 +64,16 @@ __device__ long long* g_phase_clocks;  // 8 stamps per block, set by a probe bui
 // Lanes per matrix and matrices per warp (= per block).
 template <int TMAX>
 __host__ __device__ constexpr int eigh_reg_lanes() {
-  return TMAX <= 48 ? 16 : 32;
+  return TMAX <= 32 ? 8 : (TMAX <= 48 ? 16 : 32);
 }
 template <int TMAX>
 __host__ __device__ constexpr int eigh_reg_mats() {
   return 32 / eigh_reg_lanes<TMAX>();
+}
+// Eigenvectors formed at once: two lanes each.
+template <int TMAX>
+__host__ __device__ constexpr int eigh_reg_group() {
+  return eigh_reg_lanes<TMAX>() >= 2 * kInvGroup ? kInvGroup : eigh_reg_lanes<TMAX>() / 2;
 }
 
 // Shared-memory floats per matrix: packed HV, d, e, tau, lam, p (5 TMAX), the work
@@ -76,8 +83,8 @@ __host__ __device__ constexpr int eigh_reg_mats() {
 // different banks.
 template <int TMAX>
 __host__ __device__ constexpr size_t eigh_reg_mat_floats() {
-  const size_t f = eigh_hv_floats<TMAX>() + 5 * TMAX + (size_t)2 * TMAX * kInvGroup;
-  return ((f + 31) & ~size_t(31)) + 16;
+  const size_t f = eigh_hv_floats<TMAX>() + 5 * TMAX + (size_t)2 * TMAX * eigh_reg_group<TMAX>();
+  return ((f + 31) & ~size_t(31)) + (eigh_reg_mats<TMAX>() == 4 ? 8 : 16);
 }
 template <int TMAX>
 __host__ __device__ constexpr size_t eigh_reg_smem_floats() {
@@ -387,14 +394,14 @@ __device__ __forceinline__ double mp_rank_sub(const float* lam, float unscale, i
 }
 
 // Eigenvectors of the tridiagonal for the eigenvalues lam[n - 1 - j0 - q], q < g <=
-// kInvGroup, unnormalised, entry i at Z[i * kInvGroup + q], by the L lanes of a
-// matrix, two per vector. Z and U: n x kInvGroup each.
-template <int L>
+// IG, unnormalised, entry i at Z[i * IG + q], by the L lanes of a
+// matrix, two per vector. Z and U: n x IG each.
+template <int L, int IG = kInvGroup>
 __device__ __forceinline__ void twisted_vectors(const float* d, const float* e, const float* lam, float* Z, float* U,
                                                 int n, int j0, int g, float tnorm) {
   const int l = threadIdx.x & (L - 1);
-  const int q = l & (kInvGroup - 1), down = (l / kInvGroup) & 1;  // down 0: from the top, 1: from the bottom
-  const bool on = l < 2 * kInvGroup && q < g;
+  const int q = l & (IG - 1), down = (l / IG) & 1;  // down 0: from the top, 1: from the bottom
+  const bool on = l < 2 * IG && q < g;
   const float pivtol = Num<float>::eps() * tnorm;
   float sig = on ? lam[n - 1 - j0 - q] : 0.f;
   float* F = (down ? U : Z) + q;  // e_i / pivot of this direction
@@ -409,7 +416,7 @@ __device__ __forceinline__ void twisted_vectors(const float* d, const float* e, 
         const float ei = e[i], dn = d[down ? i : i + 1] - sig;
         if (fabsf(D) < pivtol) D = D < 0.f ? -pivtol : pivtol;
         const float r = __fdividef(ei, D);
-        F[i * kInvGroup] = r;
+        F[i * IG] = r;
         D = fmaf(-ei, r, dn);
       }
     }
@@ -421,8 +428,8 @@ __device__ __forceinline__ void twisted_vectors(const float* d, const float* e, 
 #pragma unroll 4
       for (int r = down; r < n; r += 2) {
         float gr = d[r] - sig;
-        if (r > 0) gr = fmaf(-e[r - 1], Z[(r - 1) * kInvGroup + q], gr);
-        if (r < n - 1) gr = fmaf(-e[r], U[r * kInvGroup + q], gr);
+        if (r > 0) gr = fmaf(-e[r - 1], Z[(r - 1) * IG + q], gr);
+        if (r < n - 1) gr = fmaf(-e[r], U[r * IG + q], gr);
         if (fabsf(gr) < best) {
           best = fabsf(gr);
           gam = gr;
@@ -431,8 +438,8 @@ __device__ __forceinline__ void twisted_vectors(const float* d, const float* e, 
       }
     }
     {
-      const float ob = __shfl_xor_sync(0xffffffffu, best, kInvGroup), og = __shfl_xor_sync(0xffffffffu, gam, kInvGroup);
-      const int oa = __shfl_xor_sync(0xffffffffu, at, kInvGroup);
+      const float ob = __shfl_xor_sync(0xffffffffu, best, IG), og = __shfl_xor_sync(0xffffffffu, gam, IG);
+      const int oa = __shfl_xor_sync(0xffffffffu, at, IG);
       if (ob < best || (ob == best && oa < at)) {
         best = ob;
         gam = og;
@@ -442,24 +449,24 @@ __device__ __forceinline__ void twisted_vectors(const float* d, const float* e, 
     float z = 1.f, s2 = 0.f;
     if (on) {
       if (down == 0) {
-        if (pass == 1) Z[at * kInvGroup + q] = 1.f;  // (the bottom lane writes below this row)
+        if (pass == 1) Z[at * IG + q] = 1.f;  // (the bottom lane writes below this row)
 #pragma unroll 4
         for (int i = at - 1; i >= 0; --i) {
-          z = -Z[i * kInvGroup + q] * z;
+          z = -Z[i * IG + q] * z;
           s2 = fmaf(z, z, s2);
-          if (pass == 1) Z[i * kInvGroup + q] = z;
+          if (pass == 1) Z[i * IG + q] = z;
         }
       } else {
 #pragma unroll 4
         for (int i = at; i < n - 1; ++i) {
-          z = -U[i * kInvGroup + q] * z;
+          z = -U[i * IG + q] * z;
           s2 = fmaf(z, z, s2);
-          if (pass == 1) Z[(i + 1) * kInvGroup + q] = z;
+          if (pass == 1) Z[(i + 1) * IG + q] = z;
         }
       }
     }
     if (pass == 0) {
-      s2 = 1.f + s2 + __shfl_xor_sync(0xffffffffu, s2, kInvGroup);
+      s2 = 1.f + s2 + __shfl_xor_sync(0xffffffffu, s2, IG);
       // the correction stays within the eigenvalue's own tolerance
       const float cor = __fdividef(gam, s2), lim = 2.f * pivtol;
       sig += fminf(fmaxf(cor, -lim), lim);
@@ -473,13 +480,24 @@ __device__ __forceinline__ void twisted_vectors(const float* d, const float* e, 
 // vectors before them, which are read from the output ``V``; then written there.
 // gmax >= g: vectors of the fullest matrix of the warp (one with fewer works on
 // zeros).
-template <int L, int R>
-__device__ __forceinline__ void gram_schmidt(float2 (&y)[R][kInvGroup / 2], float* V, int n, int j0, int g, int gmax,
-                                             bool mine) {
+// Returns whether the float32 vectors could not tell a kept eigenvalue from an earlier
+// one: what the projections leave of its vector is below a tenth in length. Two
+// eigenvalues that agree to the shifts' errors can start both vectors from the same
+// row, and the rest would be round-off. An eigenvalue below kRoundOff of the norm is
+// round-off itself, and any orthonormal vector does: of a rank-deficient matrix the
+// tail of the tridiagonal is round-off, its vectors are unit vectors that coincide,
+// and nothing is left of one after two rounds; it goes on from vectors of signs.
+constexpr float kParallel = 1e-2f;
+constexpr float kRoundOff = 0x1p-21f;
+constexpr int kGsRounds = 10;
+template <int L, int R, int IG = kInvGroup>
+__device__ __forceinline__ bool gram_schmidt(float2 (&y)[R][IG / 2], float* V, const float* lam, float tnorm, int n,
+                                             int j0, int g, int gmax, bool mine) {
+  bool lost = false;
   const int l = threadIdx.x & (L - 1);
   auto vq = [&](int ri, int q) -> float& { return (q & 1) ? y[ri][q / 2].y : y[ri][q / 2].x; };
 #pragma unroll
-  for (int q = 0; q < kInvGroup; ++q) {
+  for (int q = 0; q < IG; ++q) {
     if (q >= gmax) continue;
     auto norm2 = [&]() {
       float s_ = 0.f;
@@ -495,10 +513,21 @@ __device__ __forceinline__ void gram_schmidt(float2 (&y)[R][kInvGroup / 2], floa
 #pragma unroll
       for (int ri = 0; ri < R; ++ri) vq(ri, q) = fmaf(-dot, w[ri], vq(ri, q));
     };
-    const float before = norm2();
-    bool on = true;  // this matrix takes part
+    float before = norm2();
+    bool on = q < g;  // this matrix takes part
 #pragma unroll 1
-    for (int round = 0; round < 2; ++round) {
+    for (int round = 0; round < kGsRounds; ++round) {
+      if (round >= 2) {  // nothing but round-off was left: another start
+#pragma unroll
+        for (int ri = 0; ri < R; ++ri) {
+          const unsigned r = l + L * ri;
+          unsigned h = (r + 1u) * 0x9E3779B1u ^ (unsigned)(j0 + q + 128 * round) * 0x85EBCA6Bu;
+          h = (h ^ (h >> 15)) * 0xC2B2AE35u;
+          const float s_ = (h >> 16) & 1u ? 1.f : -1.f;
+          if (on) vq(ri, q) = (int)r < n && q < g ? s_ : 0.f;
+        }
+        before = on ? (float)n : before;
+      }
       for (int i = 0; i < j0; ++i) {  // earlier chunks, from the output
         float w[R];
 #pragma unroll
@@ -518,13 +547,15 @@ __device__ __forceinline__ void gram_schmidt(float2 (&y)[R][kInvGroup / 2], floa
       for (int ri = 0; ri < R; ++ri) vq(ri, q) *= inv;
       // little left of it (nearly parallel to the earlier ones): once more, from
       // the normalised rest
-      on = after < 1e-3f * before;
+      if (round == 0 && on && after < kParallel * before) lost |= lam[n - 1 - j0 - q] > kRoundOff * tnorm;
+      on &= after < 1e-3f * before;
+      before = 1.f;
       if (!__any_sync(0xffffffffu, on)) break;
     }
   }
   if (mine) {
 #pragma unroll
-    for (int q = 0; q < kInvGroup; ++q)
+    for (int q = 0; q < IG; ++q)
       if (q < g)
 #pragma unroll
         for (int ri = 0; ri < R; ++ri) {
@@ -532,6 +563,7 @@ __device__ __forceinline__ void gram_schmidt(float2 (&y)[R][kInvGroup / 2], floa
           if (r < n) V[(long long)(j0 + q) * n + r] = vq(ri, q);
         }
   }
+  return lost;
 }
 
 // Body of one warp's matrices ``b0``, b0 + 1 (the launch's patch index, below nmat;
@@ -542,7 +574,12 @@ __device__ __forceinline__ void eigh_reg_body(const float* gram, float* vecs, fl
                                               float* __restrict__ sig2, int n, int nvox, long long patch0,
                                               int* __restrict__ refine_count, int* __restrict__ refine_ids,
                                               long long b0, long long nmat) {
-  constexpr int L = eigh_reg_lanes<TMAX>(), R = TMAX / L, NG = TMAX / 4;
+  constexpr int L = eigh_reg_lanes<TMAX>(), R = TMAX / L, NG = TMAX / 4, IG = eigh_reg_group<TMAX>();
+  // Whether the reflector's next column groups are read two groups ahead: a switch's
+  // labels keep the compiler from moving a load up. Eigensolve phase off / on: 37392
+  // matrices at T = 64 3.07 / 2.91 ms, 12600 at T = 48 0.731 / 0.745 (out of registers;
+  // one matrix 105 / 97 us), 372416 at T = 32 5.21 / 5.21.
+  constexpr bool PF = TMAX > 48;
   extern __shared__ __align__(16) float sr[];
   const int lane = threadIdx.x & 31, l = lane & (L - 1);
   const bool mine = b0 + lane / L < nmat;  // the last warp's second half may have no matrix of its own
@@ -674,14 +711,18 @@ __device__ __forceinline__ void eigh_reg_body(const float* gram, float* vecs, fl
     float2 s01[R], s23[R];
 #pragma unroll
     for (int ri = 0; ri < R; ++ri) s01[ri] = s23[ri] = make_float2(0.f, 0.f);
+    float4 ve, vo;
+    if constexpr (PF) ve = hv4[(j4lo + 1) & ~1], vo = hv4[j4lo | 1];
 #define LRD_MV(J)                                                    \
   case J:                                                            \
     if constexpr (J < NG) {                                          \
-      const float4 v4 = hv4[J];                                      \
+      float4& v4 = (J & 1) ? vo : ve;                                \
+      if constexpr (!PF) v4 = hv4[J];                                \
       _Pragma("unroll") for (int ri = 0; ri < R; ++ri) {             \
         fma2(s01[ri], a[ri][2 * J], make_float2(v4.x, v4.y));        \
         fma2(s23[ri], a[ri][2 * J + 1], make_float2(v4.z, v4.w));    \
       }                                                              \
+      if constexpr (PF && J + 2 < NG) v4 = hv4[J + 2];               \
     }
     switch (j4lo) {
       LRD_MV(0) LRD_MV(1) LRD_MV(2) LRD_MV(3) LRD_MV(4) LRD_MV(5) LRD_MV(6) LRD_MV(7)
@@ -708,16 +749,25 @@ __device__ __forceinline__ void eigh_reg_body(const float* gram, float* vecs, fl
       mv[ri] = make_float2(-v[ri], -v[ri]);
       mc[ri] = make_float2(-c, -c);
     }
+    float4 pe, po;
+    if constexpr (PF) {
+      ve = hv4[(j4lo + 1) & ~1], vo = hv4[j4lo | 1];
+      pe = ps4[(j4lo + 1) & ~1], po = ps4[j4lo | 1];
+    }
 #define LRD_UPD(J)                                                   \
   case J:                                                            \
     if constexpr (J < NG) {                                          \
-      const float4 v4 = hv4[J];                                      \
-      const float4 p4 = ps4[J];                                      \
+      float4 &v4 = (J & 1) ? vo : ve, &p4 = (J & 1) ? po : pe;       \
+      if constexpr (!PF) v4 = hv4[J], p4 = ps4[J];                   \
       _Pragma("unroll") for (int ri = 0; ri < R; ++ri) {             \
         fma2(a[ri][2 * J], mc[ri], make_float2(v4.x, v4.y));         \
         fma2(a[ri][2 * J + 1], mc[ri], make_float2(v4.z, v4.w));     \
         fma2(a[ri][2 * J], mv[ri], make_float2(p4.x, p4.y));         \
         fma2(a[ri][2 * J + 1], mv[ri], make_float2(p4.z, p4.w));     \
+      }                                                              \
+      if constexpr (PF && J + 2 < NG) {                              \
+        v4 = hv4[J + 2];                                             \
+        p4 = ps4[J + 2];                                             \
       }                                                              \
     }
     switch (j4lo) {
@@ -749,47 +799,39 @@ __device__ __forceinline__ void eigh_reg_body(const float* gram, float* vecs, fl
   LRD_STAMP(3);
   int p;
   const double margin = mp_rank_sub<L>(lam, unscale, n, nvox, W, p, (sig2 && mine) ? sig2 + b : nullptr);
+  // queued for float64: a near-tie, or a vector that Gram-Schmidt finds lost
+  bool queue = margin < kRefineTol;
   if (l == 0 && mine) {
     ranks[b] = p;
     wgt[b] = (float)(1.0 / (2.0 + (double)p));
-    // Queued for float64: a near-tie, or two kept eigenvalues too close for the
-    // float32 vectors to tell apart (both twisted factorisations could give the
-    // same vector). Below 64 eps of the norm they are round-off themselves, and
-    // any orthonormal vectors do.
-    bool queue = margin < kRefineTol;
-    for (int j = 1; j < p; ++j) {
-      const float lo = lam[n - 1 - j], hi = lam[n - j];
-      queue |= hi - lo < 4.f * Num<float>::eps() * tnorm && lo > 64.f * Num<float>::eps() * tnorm;
-    }
-    if (refine_count != nullptr && queue) refine_ids[atomicAdd(refine_count, 1)] = (int)(patch0 + b);
   }
   if (lam_out != nullptr && mine)
     for (int i = l; i < n; i += L) lam_out[b * n + i] = lam[i] * unscale;
   LRD_STAMP(4);
   const int pmax = (int)__reduce_max_sync(0xffffffffu, (unsigned)p);
 
-  // ---- top-p eigenvectors, 8 at a time -------------------------------------------
+  // ---- top-p eigenvectors, IG at a time -------------------------------------------
   float* V = vecs + b * (long long)n * n;
   float* Z = W;
-  float* U = W + TMAX * kInvGroup;
+  float* U = W + TMAX * IG;
 #pragma unroll 1
-  for (int j0 = 0; j0 < pmax; j0 += kInvGroup) {
-    const int g = min(kInvGroup, p - j0);  // <= 0: this matrix has no more
+  for (int j0 = 0; j0 < pmax; j0 += IG) {
+    const int g = min(IG, p - j0);  // <= 0: this matrix has no more
     __syncwarp();
-    twisted_vectors<L>(d, e, lam, Z, U, n, j0, g, tnorm);
+    twisted_vectors<L, IG>(d, e, lam, Z, U, n, j0, g, tnorm);
     LRD_STAMP(5);
     // row-distributed: y[ri][q / 2] = vectors q, q + 1, row l + L ri
-    float2 y[R][kInvGroup / 2];
+    float2 y[R][IG / 2];
 #pragma unroll
     for (int ri = 0; ri < R; ++ri) {
       const int r = l + L * ri;
 #pragma unroll
-      for (int q = 0; q < kInvGroup; q += 2) {
-        const float2 z = *reinterpret_cast<const float2*>(Z + r * kInvGroup + q);
+      for (int q = 0; q < IG; q += 2) {
+        const float2 z = *reinterpret_cast<const float2*>(Z + r * IG + q);
         y[ri][q / 2] = make_float2(r < n && q < g ? z.x : 0.f, r < n && q + 1 < g ? z.y : 0.f);
       }
     }
-    // back-transform x = H(0) ... H(n-3) y, on the first 2 G vectors of the chunk
+    // back-transform x = H(0) ... H(n-3) y, on the first 2 GP vectors of the chunk
     auto back_transform = [&](auto gtag) {
       constexpr int GP = decltype(gtag)::value;
       int hb = hbase;  // end of the packed rows
@@ -821,21 +863,22 @@ __device__ __forceinline__ void eigh_reg_body(const float* gram, float* vecs, fl
         }
       }
     };
-    if (pmax - j0 <= 4)
+    if (IG == 4 || pmax - j0 <= 4)
       back_transform(IntTag<2>{});
     else
-      back_transform(IntTag<4>{});
+      back_transform(IntTag<IG / 2>{});
     LRD_STAMP(6);
-    gram_schmidt<L, R>(y, V, n, j0, g, min(kInvGroup, pmax - j0), mine);
+    queue |= gram_schmidt<L, R, IG>(y, V, lam, tnorm, n, j0, g, min(IG, pmax - j0), mine);
     __syncwarp();
   }
+  if (l == 0 && mine && refine_count != nullptr && queue) refine_ids[atomicAdd(refine_count, 1)] = (int)(patch0 + b);
   LRD_STAMP(7);
 }
 
 // Warps per SM by the registers the rows need (R TMAX and about 50 more).
 template <int TMAX>
 __host__ __device__ constexpr int eigh_reg_min_blocks() {
-  return TMAX <= 32 ? 16 : 12;
+  return 12;
 }
 
 template <int TMAX>

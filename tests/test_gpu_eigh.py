@@ -96,3 +96,36 @@ def test_equal_signal_eigenvalues(cuda_ok, T):
     assert rel_l2(out.cpu().numpy(), ref64) <= 1e-6
     plain = api.denoise(d, patch, 2)
     assert rel_l2(plain.cpu().numpy(), ref) <= 1e-6
+
+
+@pytest.mark.parametrize("T", [24, 32, 48, 64, 96, 127])
+def test_round_off_vectors_are_orthonormal(cuda_ok, T):
+    """Two equal components over round-off: the tridiagonal's tail vanishes, many kept
+    eigenvalues are round-off, and their vectors coincide before they are made
+    orthogonal. A projection leaves at least 0.03 of a vector, so T dot products of
+    T terms, rounded by T 2^-24 each, put V^T V at most 2 T 2^-24 / 0.03 from 1; the
+    two components' span moves by the reduction's T 2^-24 a few times over."""
+    shape, patch = (8, 8, 6, T), (8, 8, 4)
+    rng = np.random.default_rng(1)
+    x, y, z = np.meshgrid(*(np.arange(s) for s in shape[:3]), indexing="ij")
+    k = 2 * np.pi * np.arange(T) / T
+    vol = ((-1.0) ** x)[..., None] * np.sin(3 * k) + ((-1.0) ** y)[..., None] * np.cos(3 * k)
+    vol = (vol + 1e-6 * rng.standard_normal(shape)).astype(np.float32)
+    plan = api.get_plan(shape, patch, 2)
+    P = plan.n_patches
+    ws = torch.empty(plan.workspace_bytes, dtype=torch.uint8, device="cuda")
+    s = torch.cuda.current_stream().cuda_stream
+    G = torch.empty(P, T, T, device="cuda")
+    d = torch.from_numpy(vol).cuda()
+    plan.stage_gram(d.data_ptr(), G.data_ptr(), ws.data_ptr(), s)
+    lam, vecs = torch.empty(P, T, device="cuda"), torch.empty(P, T, T, device="cuda")
+    ranks = torch.empty(P, dtype=torch.int32, device="cuda")
+    plan.stage_eigh(G.data_ptr(), lam.data_ptr(), vecs.data_ptr(), ranks.data_ptr(), ws.data_ptr(), s)
+    torch.cuda.synchronize()
+    for i in range(P):
+        p = int(ranks[i])
+        assert p >= 2
+        V = vecs[i].cpu().numpy().reshape(-1)[: T * p].reshape(p, T).T.astype(np.float64)
+        assert np.abs(V.T @ V - np.eye(p)).max() <= 2 * T * 2.0 ** -24 / 0.03
+        U = np.linalg.eigh(G[i].cpu().numpy().astype(np.float64))[1][:, -2:]
+        assert np.linalg.norm(U - V[:, :2] @ (V[:, :2].T @ U)) <= 8 * T * 2.0 ** -24
