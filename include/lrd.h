@@ -141,7 +141,9 @@ int lrd_denoise(const lrd_plan* plan, const float* d_vol, float* d_out, int32_t*
  * ``stream``, its reconstruction on another plan stream, and finished output
  * planes copy out while later slabs compute (pinned host buffers make the
  * copies asynchronous). Results are identical to lrd_denoise's. The plan's
- * streams and events make this one call at a time per plan. */
+ * streams and events make this one call at a time per plan. Pageable input of
+ * 32 MiB or more goes through 16 MiB of pinned memory that the plan keeps, filled
+ * by threads that live for the call. */
 int lrd_denoise_host(const lrd_plan* plan, const float* h_vol, float* h_out, int32_t* h_ranks,
                      float* d_in, float* d_out, int32_t* d_ranks, void* d_workspace,
                      void* stream);

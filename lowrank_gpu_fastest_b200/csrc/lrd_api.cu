@@ -23,6 +23,7 @@
 #include "gram.cuh"
 #include "gram_tc.cuh"
 #include "gram_z.cuh"
+#include "host_stage.cuh"
 #include "lrd_common.cuh"
 #include "recon.cuh"
 #include "recon_tc.cuh"
@@ -113,6 +114,7 @@ struct lrd_plan {
   // the enqueue of a call holds the mutex (the streams and events are shared)
   int dev_slabs = 1;
   mutable std::mutex pipe_mu;
+  mutable lrd::StageRing stage;  // pinned slots for pageable inputs (held with pipe_mu)
   // measurement hook: a ring of per-call phase events
   bool profiling = false;
   int prof_calls = 0;
@@ -1191,14 +1193,35 @@ int lrd_denoise_host(const lrd_plan* P, const float* h_vol, float* h_out, int32_
   // volume's slabs would be launch- and event-bound
   const long long vbytes = (long long)sizeof(float) * P->nvox * g.nt;
   const int S = std::max(1, std::min<int>({kIoSlabsUsed, g.ncx, (int)((vbytes + kIoSlabBytes - 1) / kIoSlabBytes)}));
+  auto planes_for = [&](int s) {  // input planes slabs 0 ... s need
+    return s == S - 1 ? g.nx : std::min(g.nx, P->h_corner_x[slab_end(s, S, g.ncx) - 1] + g.px);
+  };
+  // pageable input goes by way of pinned slots (the driver's own staging where that
+  // cannot be set up)
+  std::unique_ptr<lrd::StagedCopy> staged;
+  if (vbytes >= lrd::kStageMinBytes) {
+    cudaPointerAttributes at{};
+    if (cudaPointerGetAttributes(&at, h_vol) != cudaSuccess) {
+      cudaGetLastError();
+    } else if (at.type == cudaMemoryTypeUnregistered && P->stage.make()) {
+      try {
+        std::vector<size_t> ends;
+        for (int s = 0; s < S; ++s) ends.push_back(sizeof(float) * (size_t)planes_for(s) * plane);
+        staged = std::make_unique<lrd::StagedCopy>(P->stage, h_vol, ends, P->device);
+      } catch (...) {
+      }
+    }
+  }
   int planes_in = 0, ci_done = 0, bx_done = 0;
   const long long colz = (long long)g.ncy, patz = (long long)g.ncy * g.ncz, brz = (long long)g.nby * g.nbz;
   for (int s = 0; s < S; ++s) {
     const int ci_end = slab_end(s, S, g.ncx);
     const bool lastslab = s == S - 1;
-    const int x_need = lastslab ? g.nx : std::min(g.nx, P->h_corner_x[ci_end - 1] + g.px);
+    const int x_need = planes_for(s);
     cudaStream_t prep = P->io_prep[s % 3];
-    if (x_need > planes_in)
+    if (staged)
+      LRD_CUDA(staged->send(d_in, sizeof(float) * (size_t)x_need * plane, P->io_in));
+    else if (x_need > planes_in)
       LRD_CUDA(cudaMemcpyAsync(d_in + planes_in * plane, h_vol + planes_in * plane,
                                sizeof(float) * (size_t)(x_need - planes_in) * plane, cudaMemcpyHostToDevice,
                                P->io_in));
