@@ -132,7 +132,7 @@ constexpr int kIoSlabs = 16;     // event capacity of the host-buffer pipeline
 // x-slabs the host-buffer pipeline uses (about 3.5 MiB of input each, at most
 // this many). Measured e2e at 96x96x48x48 / 11^3 / stride 3 on B200 (ms), one
 // reconstruction stream: 4 slabs 4.73, 6 4.74, 8 4.62, 10 4.55, 12 4.62, 16
-// 5.05; with the current kernels 8 3.61, 10 3.60, 12 3.62; two alternating
+// 5.05; then 8 3.61, 10 3.60, 12 3.62; two alternating
 // reconstruction streams: 8 3.61, 10 3.51, 12 3.48; and two / three / four
 // solve streams: 12 slabs 3.48 / 3.48 / 3.60, 16 3.49 / 3.38 / 3.53, 20
 // 3.63 / 3.45 / 3.65, 24 3.90 / 3.60 / 3.73. At 48x48x24x48 (10 MiB), three
@@ -620,7 +620,7 @@ int validate_problem(const lrd_problem* pr) {
 // CTA). Without either, frame counts the warp kernel is built for take it
 // (``warp``; recon_warp_brick()).
 // Measured on B200, reconstruction ms, 96x96x48x48 / 11^3 / stride 3:
-// brick kernel (3x3x3, 2 threads per voxel) 1.22 -> warp kernel (see DESIGN).
+// brick kernel (3x3x3, 2 threads per voxel) 1.22 -> warp kernel 0.83.
 int pick_layout(const lrd_problem* pr, const int dims[3], const int pat[3], const std::vector<int32_t> corners[3],
                 int& rsplit, int& rtpt, int best[3], bool* warp = nullptr, bool* tc = nullptr) {
   if (warp) *warp = false;
