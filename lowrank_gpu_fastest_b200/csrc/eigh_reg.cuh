@@ -33,7 +33,7 @@
 // Measured on B200 (kernel time, against one matrix per warp with bisection by the
 // quotient recurrence and inverse iteration by partial-pivoting LU): 12600 matrices
 // at T = 48 0.885 -> 0.52 ms, 372416 at T = 32 11.5 -> 5.2 (16 lanes per matrix 5.5),
-// 37392 at T = 64 4.55 -> 2.75, one matrix 105 -> 97 us. Cycles per warp at T = 48, 12 warps per SM (two matrices):
+// 37392 at T = 64 4.55 -> 2.75, one matrix 105 -> 85 us (eigh_reg_wide_kernel). Cycles per warp at T = 48, 12 warps per SM (two matrices):
 // load 9 K, reduction 128 K, eigenvalues 67 K, rank 5 K, vectors 18 K, back-transform
 // 15 K, Gram-Schmidt 4 K (one matrix per warp at 16 warps: 12 / 147 / 93 / 6 / 29 / 22 /
 // 4 K). Instruction issue 46%, three warps per scheduler: latency bounds it, the
@@ -566,20 +566,19 @@ __device__ __forceinline__ bool gram_schmidt(float2 (&y)[R][IG / 2], float* V, c
   return lost;
 }
 
-// Body of one warp's matrices ``b0``, b0 + 1 (the launch's patch index, below nmat;
-// patch patch0 + b), shared by the single-volume kernel and the packed launch.
-template <int TMAX>
+// Body of one warp's matrices ``b0``, b0 + 1, ... (the launch's patch index, below nmat;
+// patch patch0 + b), shared by the single-volume kernels and the packed launch.
+// PF: whether the reflector's next column groups are read two groups ahead: a switch's
+// labels keep the compiler from moving a load up. Eigensolve phase off / on: 37392
+// matrices at T = 64 3.07 / 2.91 ms, 12600 at T = 48 0.731 / 0.745 (out of registers;
+// eigh_reg_wide_kernel has them), 372416 at T = 32 5.21 / 5.21.
+template <int TMAX, bool PF = (TMAX > 48)>
 __device__ __forceinline__ void eigh_reg_body(const float* gram, float* vecs, float* __restrict__ lam_out,
                                               int32_t* __restrict__ ranks, float* __restrict__ wgt,
                                               float* __restrict__ sig2, int n, int nvox, long long patch0,
                                               int* __restrict__ refine_count, int* __restrict__ refine_ids,
                                               long long b0, long long nmat) {
   constexpr int L = eigh_reg_lanes<TMAX>(), R = TMAX / L, NG = TMAX / 4, IG = eigh_reg_group<TMAX>();
-  // Whether the reflector's next column groups are read two groups ahead: a switch's
-  // labels keep the compiler from moving a load up. Eigensolve phase off / on: 37392
-  // matrices at T = 64 3.07 / 2.91 ms, 12600 at T = 48 0.731 / 0.745 (out of registers;
-  // one matrix 105 / 97 us), 372416 at T = 32 5.21 / 5.21.
-  constexpr bool PF = TMAX > 48;
   extern __shared__ __align__(16) float sr[];
   const int lane = threadIdx.x & 31, l = lane & (L - 1);
   const bool mine = b0 + lane / L < nmat;  // the last warp's second half may have no matrix of its own
@@ -888,6 +887,19 @@ __global__ void __launch_bounds__(32, eigh_reg_min_blocks<TMAX>())
                     int* __restrict__ refine_count, int* __restrict__ refine_ids, long long nmat) {
   eigh_reg_body<TMAX>(gram, vecs, lam_out, ranks, wgt, sig2, n, nvox, patch0, refine_count, refine_ids,
                       (long long)blockIdx.x * eigh_reg_mats<TMAX>(), nmat);
+}
+
+// The same with eight warps per SM and the registers that gives: for launches that
+// fit the device at once, where a matrix's latency is all that counts (bit-identical
+// results; the same operations in the same order).
+constexpr int kEighWideBlocks = 8;
+template <int TMAX>
+__global__ void __launch_bounds__(32, kEighWideBlocks)
+    eigh_reg_wide_kernel(const float* gram, float* vecs, float* __restrict__ lam_out, int32_t* __restrict__ ranks,
+                         float* __restrict__ wgt, float* __restrict__ sig2, int n, int nvox, long long patch0,
+                         int* __restrict__ refine_count, int* __restrict__ refine_ids, long long nmat) {
+  eigh_reg_body<TMAX, true>(gram, vecs, lam_out, ranks, wgt, sig2, n, nvox, patch0, refine_count, refine_ids,
+                            (long long)blockIdx.x * eigh_reg_mats<TMAX>(), nmat);
 }
 
 }  // namespace lrd

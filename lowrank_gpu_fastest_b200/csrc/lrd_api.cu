@@ -281,6 +281,12 @@ const void* eigh_kernel_for(int T, bool cta, unsigned* threads = nullptr) {
   return (const void*)lrd::eigh_reg_kernel<64>;
 }
 
+// Whether small launches of this frame count have a kernel of their own.
+// Eigensolve phase on B200 at T = 48, without / with it: one matrix 0.105 / 0.085 ms, 1176
+// matrices 0.109 / 0.087. It runs where the launch fits the device at its eight warps
+// per SM; above, twelve warps hide each other's latency (12600 matrices 0.73).
+bool eigh_wide(int T, bool cta) { return !cta && T > 32 && T <= 48; }
+
 template <int TPT, int SPLIT>
 void* recon_fn(bool accurate) {
   return accurate ? (void*)lrd::recon_kernel<TPT, SPLIT, true> : (void*)lrd::recon_kernel<TPT, SPLIT, false>;
@@ -525,7 +531,10 @@ int run_eigh(const lrd_plan* P, char* ws, const float* d_gram, float* d_vecs, fl
     int tv = T, nvv = nv;
     void* eargs[] = {(void*)&gin, (void*)&vout, (void*)&lout, (void*)&r,      (void*)&w,   (void*)&s2,
                      (void*)&tv,  (void*)&nvv,  (void*)&p0v,  (void*)&rcount, (void*)&rids, (void*)&nmat};  // nmat: the warp kernels
-    cudaError_t le = cudaLaunchKernel(efn, dim3((unsigned)((nb + mats - 1) / mats)), dim3(eth), eargs, P->smem_eigh, st);
+    const long long blocks = (nb + mats - 1) / mats;
+    if (eigh_wide(T, P->eigh_cta) && blocks <= (long long)lrd::kEighWideBlocks * P->sms)
+      efn = (const void*)lrd::eigh_reg_wide_kernel<48>;
+    cudaError_t le = cudaLaunchKernel(efn, dim3((unsigned)blocks), dim3(eth), eargs, P->smem_eigh, st);
     if (le != cudaSuccess) return cuda_fail(le, "eigh kernel launch");
     int rc = launch_check("eigh kernel launch");
     if (rc) return rc;
@@ -851,6 +860,7 @@ int create_plan(const lrd_problem* pr, const std::vector<int32_t>* x_corners, lr
     }
   }
   if (!rc) rc = set_smem(eigh_kernel_for(T, P->eigh_cta), P->smem_eigh);
+  if (!rc && eigh_wide(T, P->eigh_cta)) rc = set_smem((const void*)lrd::eigh_reg_wide_kernel<48>, P->smem_eigh);
   if (!rc && P->recon_warp) rc = set_smem(recon_warp_ptr(T, pr->form != LRD_FORM_PLAIN), lrd::recon_warp_smem_bytes(T));
   if (!rc && !P->recon_tc) rc = set_smem(recon_kernel_ptr(P->tpt, P->split, false), P->smem_recon);
   if (!rc && !P->recon_tc) rc = set_smem(recon_kernel_ptr(P->tpt, P->split, true), P->smem_recon);

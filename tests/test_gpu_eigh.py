@@ -129,3 +129,15 @@ def test_round_off_vectors_are_orthonormal(cuda_ok, T):
         assert np.abs(V.T @ V - np.eye(p)).max() <= 2 * T * 2.0 ** -24 / 0.03
         U = np.linalg.eigh(G[i].cpu().numpy().astype(np.float64))[1][:, -2:]
         assert np.linalg.norm(U - V[:, :2] @ (V[:, :2].T @ U)) <= 8 * T * 2.0 ** -24
+
+
+@pytest.mark.parametrize("T", [33, 40, 48])
+def test_small_launches_agree(cuda_ok, T):
+    """A launch that fits the device at once takes another kernel: equal bit for bit to
+    the same patches in one large launch (3179 of them), with and without a remainder."""
+    rng = np.random.default_rng(T)
+    vol = torch.from_numpy(rng.standard_normal((20, 20, 14, T)).astype(np.float32)).cuda()
+    want, ranks = api.denoise(vol, (4, 4, 4), 1, return_ranks=True)
+    for batch in (97, 2000):
+        got, r = api.denoise(vol, (4, 4, 4), 1, batch=batch, return_ranks=True)
+        assert torch.equal(got, want) and torch.equal(r, ranks)
