@@ -33,7 +33,8 @@
 // Measured on B200 (kernel time, against one matrix per warp with bisection by the
 // quotient recurrence and inverse iteration by partial-pivoting LU): 12600 matrices
 // at T = 48 0.885 -> 0.52 ms, 372416 at T = 32 11.5 -> 5.2 (16 lanes per matrix 5.5),
-// 37392 at T = 64 4.55 -> 2.75, one matrix 105 -> 85 us (eigh_reg_wide_kernel). Cycles per warp at T = 48, 12 warps per SM (two matrices):
+// 37392 at T = 64 4.55 -> 2.9 (phase 3.07, with the reflector read ahead 2.89), one
+// matrix 105 -> 85 us (eigh_reg_wide_kernel). Cycles per warp at T = 48, 12 warps per SM (two matrices):
 // load 9 K, reduction 128 K, eigenvalues 67 K, rank 5 K, vectors 18 K, back-transform
 // 15 K, Gram-Schmidt 4 K (one matrix per warp at 16 warps: 12 / 147 / 93 / 6 / 29 / 22 /
 // 4 K). Instruction issue 46%, three warps per scheduler: latency bounds it, the
