@@ -50,6 +50,7 @@
 // writes NaN.
 #pragma once
 
+#include "copy_phases.h"
 #include "gram_z.cuh"  // mbarrier waits
 #include "lrd_common.cuh"
 #include "recon.cuh"
@@ -323,10 +324,9 @@ __device__ __forceinline__ void recon_warp_body(const float* __restrict__ xc, co
     }
     return n;
   };
-  unsigned phase = 0, pending = 0;  // bit b: buffer b's parity, a copy of warp 0 in flight
-  bool ok = true;                   // no wait of this warp has given up
+  CopyPhases ph;
   auto copy = [&](const ReconChunk& c, int b) {  // warp 0: the chunk's rows into buffer b
-    if (c.rows <= 0 || !ok) return;
+    if (c.rows <= 0 || !ph.ok) return;
     if (lane == 0) {
       asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
       mbar_expect_tx(bar0 + 8 * b, (uint32_t)(c.rows * T * sizeof(float)));
@@ -337,7 +337,7 @@ __device__ __forceinline__ void recon_warp_body(const float* __restrict__ xc, co
       bulk_copy(buf0 + (uint32_t)((b * ROWS + c.off) * T * sizeof(float)), vecs + pid * (T * T),
                 (uint32_t)(c.p * T * sizeof(float)), bar0 + 8 * b);
     }
-    pending |= 1u << b;
+    ph.issued(b);
   };
   const bool none = bihi < bilo || bjhi < bjlo || bkhi < bklo;  // a brick no patch touches
   ReconChunk cur{none ? bihi + 1 : bilo, bjlo, bklo, 0, 0, 0, 0, 0.f}, nxt;
@@ -353,11 +353,8 @@ __device__ __forceinline__ void recon_warp_body(const float* __restrict__ xc, co
     if (warp == 0) copy(nxt, b ^ 1);
     ReconChunk then = after(nxt);
     fetch(then);
-    if (cur.rows > 0) {
-      if (ok) ok = __all_sync(0xffffffffu, mbar_wait_bounded(bar0 + 8 * b, (phase >> b) & 1, status));
-      if (ok) pending &= ~(1u << b);
-      phase ^= 1u << b;
-    }
+    if (cur.rows > 0 && ph.ok)
+      ph.waited(b, __all_sync(0xffffffffu, mbar_wait_bounded(bar0 + 8 * b, ph.parity(b), status)));
     if (cur.j >= jlo && cur.j <= jhi) {  // (a warp's two x are the brick's)
       const bool cxy = cur.i >= cxlo && cur.i <= cxhi && cur.j >= cylo && cur.j <= cyhi;
       if (cur.rows < 0) {  // its rows straight from global memory
@@ -404,14 +401,14 @@ __device__ __forceinline__ void recon_warp_body(const float* __restrict__ xc, co
   }
   // a wait of warp 0 gave up: its copies still in flight land (or time out) before
   // the CTA's shared memory is freed
-  if (warp == 0 && lane == 0 && !ok)
+  if (warp == 0 && lane == 0 && !ph.ok)
     for (int b = 0; b < 2; ++b)
-      if ((pending >> b) & 1) mbar_wait_bounded(bar0 + 8 * b, (phase >> b) & 1, status);
+      if (ph.in_flight(b)) mbar_wait_bounded(bar0 + 8 * b, ph.parity(b), status);
 
 #pragma unroll
   for (int v = 0; v < NV; ++v) {
     if (!valid[v]) continue;
-    if (!ok) {  // rows that never came: no caller can take the result for one
+    if (!ph.ok) {  // rows that never came: no caller can take the result for one
       m[v] = wacc[v] = __int_as_float(0x7fffffff);
       wacc64[v] = (double)m[v];
     }
@@ -439,7 +436,7 @@ __device__ __forceinline__ void recon_warp_body(const float* __restrict__ xc, co
         op[u] = make_float4((float)(mm + acc64[v][4 * u + 0] * inv), (float)(mm + acc64[v][4 * u + 1] * inv),
                             (float)(mm + acc64[v][4 * u + 2] * inv), (float)(mm + acc64[v][4 * u + 3] * inv));
     } else {
-      const float den = ok ? fmaxf(wacc[v], 1e-12f) : wacc[v];
+      const float den = ph.ok ? fmaxf(wacc[v], 1e-12f) : wacc[v];
 #pragma unroll
       for (int u = 0; u < Q4; ++u)
         op[u] = make_float4(__fdiv_rn(acc[v][2 * u].x, den), __fdiv_rn(acc[v][2 * u].y, den),
