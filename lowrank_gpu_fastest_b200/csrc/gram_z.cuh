@@ -26,10 +26,10 @@
 // shared memory and which ran a CTA per patch, 68.1 -> 10.2.
 //
 // Planes that lie in the same windows (two of three at 11^3 / stride 3) are summed
-// in registers; at the last of them the KS lanes' partial sums are combined by
-// halving exchanges and added to the windows in float32, and a window is written
-// out (and its slot cleared) after its last plane. The K = px*py*pz sum therefore
-// rounds as a blocked sum: rows of a plane group, lanes, window.
+// in registers, at most gramz_group() of them; at the last the KS lanes' partial sums are
+// combined by halving exchanges and added to the windows in float32, and a window is
+// written out (and its slot cleared) after its last plane. The K = px*py*pz sum
+// therefore rounds as a blocked sum: rows of a plane group, lanes, window.
 // A frame count that is not a multiple of 4 has the rows of its centred volume padded
 // to one with zeros (TMA strides are multiples of 16 bytes), and its windows add
 // without rounding (gramz_exact): with a CTA per patch 61x53x37x65 / 7^3 / stride 2
@@ -135,6 +135,22 @@ __host__ __device__ inline int gramz_threads(int T, int ks) {
   return 32 * ((gramz_cta_blocks(T, ks) + per_warp - 1) / per_warp);
 }
 
+// Planes of a group, so that a lane's chain of additions has an end: without a limit a
+// patch that no window cuts (stride at or beyond its side, a volume one patch deep) was
+// one chain, and the Gram twice as far from float64. Relative error of the Gram (random
+// centred rows, rms, over that of planes summed one by one with half as many lanes a
+// block; windows in float64 where they carry two words here) without a limit and with 2
+// / 3 / 4 planes: stride = side, 11^3 at T = 48 1.26, 0.78 / 0.76 / 0.69, T = 64 2.04, 0.75 / 0.79 /
+// 0.80, T = 96 2.03, 0.73 / 0.79 / 0.80, T = 65 2.65, 0.69 / 0.86 / 1.06; 7^3 at T = 64 1.23, 0.79 /
+// 0.88 / 0.84, T = 31 1.75, 0.80 / 0.98 / 1.15; 15^3 at T = 96 2.72, 0.69 / 0.79 / 0.82; two lanes a
+// block, 11^3 at T = 64 3.76, 0.89 / 1.15 / 1.25. A flush has its price (Gram ms without a
+// limit, and with 2 / 3 / 4): 96x96x48x48 / 11^3 / stride 3 0.528, 0.553 / 0.530 / 0.530 (groups
+// of one and two planes, three at the volume's ends), stride 11 0.072, 0.083 / 0.078 / 0.076.
+template <int KS, bool EXACT>
+__host__ __device__ constexpr int gramz_group() {
+  return EXACT || KS == 2 ? 2 : 3;
+}
+
 // Dynamic shared memory: two plane slots, ``ring`` window accumulators (64 floats
 // per block, twice that where they carry their rounding errors), two mbarriers.
 __host__ __device__ inline size_t gramz_smem_bytes(int px, int py, int T, int ks, int ring) {
@@ -161,8 +177,8 @@ __device__ __forceinline__ float joined(float hi, float lo) { return lo == lo ? 
 // min(windows active at a plane, windows of the unit) <= ring), so a launch
 // whose last wave would hold a few whole columns spreads that tail over many
 // SMs, and a ring that does not fit shared memory is cut to one that does. The
-// planes are grouped by the column's windows, not the unit's, so the result
-// does not depend on the cut. ``col0`` = first column (x-major index
+// planes are grouped by the column's windows, not the unit's, and a unit starts and
+// ends with a group, so the result does not depend on the cut. ``col0`` = first column (x-major index
 // ci * ncy + cj); ``gram`` points at the Gram block of the launch's first
 // patch (patch index col0 * ncz).
 // Body of one CTA (index ``cta``); ``xmap`` points at the tensor map (a kernel
@@ -236,6 +252,7 @@ __device__ __forceinline__ void gram_z_body(const CUtensorMap* xmap, float* __re
 #pragma unroll
     for (int v = 0; v < 4; ++v) acc[u][v] = make_float2(0.f, 0.f);
   int nlo = tab.cover[2][2 * zlo], nhi = tab.cover[2][2 * zlo + 1];
+  int held = 0;  // planes summed in acc
   for (int z = zlo; z <= zhi; ++z) {
     const int slot = (z - zlo) & 1;
     // Each slot's barrier has at most one phase pending: plane z + 1 goes into
@@ -283,9 +300,10 @@ __device__ __forceinline__ void gram_z_body(const CUtensorMap* xmap, float* __re
       return;
     }
     if (klo > khi) continue;
-    // Planes in the same windows are summed together; the sum goes to the
-    // windows at the last of them (a window starts and ends at such a break).
-    if (z < zhi && nlo == clo && nhi == chi) continue;
+    // Planes in the same windows are summed together, up to gramz_group(); the sum goes
+    // to the windows at the last of them (a window starts and ends at such a break).
+    if (++held < gramz_group<KS, EXACT>() && z < zhi && nlo == clo && nhi == chi) continue;
+    held = 0;
     // halving exchanges over the KS lanes of a block: each step a lane keeps half
     // of its rows and adds its partner's copies of them
     float2 mine[NR][4];
