@@ -3,18 +3,20 @@ and threads per voxel, the column Gram's voxel-row split, and the
 eigensolver's matrix-per-warp or matrix-per-CTA schedule.
 
 Brick (0, 0, 0) with split 0, gram_split 0 and eigh_block 0 are the plan's
-own choices: the warp kernel (one warp per 2x2x2 voxel block) for the frame
-counts it is built for, else the brick kernel with the cost model's brick;
+own choices: the warp kernel (two warps per brick of 2x2x8 or 2x2x4 voxels) for
+the frame counts it is built for, else the brick kernel with the cost model's brick;
 the Gram split measured best per frame count; one warp per matrix up to
 T = 64.
 
 Each phase is tuned on its own phase time (the library's phase events, mean
 of ``reps`` warm calls) on a synthetic volume of the problem's shape: first
 the reconstruction over a candidate set of bricks and splits, then the Gram
-split over 1, 2, 4 (column Gram only), then the eigensolver schedule (T <= 64:
-warp or CTA). Results are cached per (GPU architecture, frames, patch,
-stride, form) in a JSON file (``LRD_TUNE_CACHE``, default
-``~/.cache/lowrank_gpu_fastest_b200/tune.json``). The reconstruction choices
+split over 1, 2, 4 (2, 4 or 8 threads per block; column Gram only), then the
+eigensolver schedule (T <= 64: warp or CTA). Results are cached per (GPU
+architecture, frames, patch, stride, form) in a JSON file (``LRD_TUNE_CACHE``,
+default ``~/.cache/lowrank_gpu_fastest_b200/tune.json``), under names that carry ``KERNELS``:
+what a package with other kernels has stored is neither used nor replaced. The
+reconstruction choices
 give bit-identical output; the Gram split and the eigensolver schedule
 change the float32 rounding of the Gram and the eigenvalues (the ranks stay
 the same: near-ties are decided in float64 from the input).
@@ -27,6 +29,11 @@ import os
 import threading
 
 import numpy as np
+
+# What the choices on disk were timed on and mean; raised with every change of either
+# (gram_split n was n threads per 4x4 block of the Gram before it was 2n per 8x8
+# block, and each phase's kernel was replaced).
+KERNELS = 3
 
 _lock = threading.Lock()
 _mem: dict = {}
@@ -69,6 +76,17 @@ def _choice(d) -> dict:
                 gram_split=int(d.get("gram_split", 0)), eigh_block=int(d.get("eigh_block", 0)))
 
 
+def _slot(k: str) -> str:
+    """The name under which the choice for key ``k`` is on disk."""
+    return f"{k}|kernels{KERNELS}"
+
+
+def _stored(k: str):
+    """The choice on disk for key ``k`` (None: none on these kernels)."""
+    e = _load().get(_slot(k))
+    return None if e is None else _choice(e)
+
+
 def candidates(T: int, patch, stride: int):
     """Bricks near the stride lattice, two thread layouts, 27..256 threads."""
     s = max(1, int(stride))
@@ -109,10 +127,10 @@ def tune(shape, patch=(11, 11, 11), stride=3, form="plain", device=None, max_can
         if not force:
             if k in _mem:
                 return dict(_mem[k])
-            disk = _load()
-            if k in disk:
-                _mem[k] = _choice(disk[k])
-                return dict(_mem[k])
+            stored = _stored(k)
+            if stored is not None:
+                _mem[k] = stored
+                return dict(stored)
 
     def slots(b):
         tot = 1.0
@@ -128,8 +146,8 @@ def tune(shape, patch=(11, 11, 11), stride=3, form="plain", device=None, max_can
 
     cands = candidates(T, patch, stride)
     cands.sort(key=lambda c: slots(c[0]) * c[1] / max(1, min(4, c[1])))
-    # the plan's own choice first (brick and split 0: the warp-per-2x2x2-block
-    # kernel where it is built for T, else the cost model's brick)
+    # the plan's own choice first (brick and split 0: the warp kernel where it is
+    # built for T, else the cost model's brick)
     cands = [((0, 0, 0), 0)] + cands[:max_candidates]
     vol, _ = make_phantom_lowrank(tuple(int(v) for v in shape), seed=7)
     timed = {"recon": [], "gram": [], "eigh_mp": []}
@@ -188,8 +206,8 @@ def tune(shape, patch=(11, 11, 11), stride=3, form="plain", device=None, max_can
     with _lock:
         _mem[k] = dict(choice)
         disk = _load()
-        disk[k] = {"brick": list(choice["brick"]), "split": choice["split"], "gram_split": choice["gram_split"],
-                   "eigh_block": choice["eigh_block"], "recon_ms": best_ms, "timed": timed}
+        disk[_slot(k)] = {"brick": list(choice["brick"]), "split": choice["split"], "gram_split": choice["gram_split"],
+                          "eigh_block": choice["eigh_block"], "recon_ms": best_ms, "timed": timed}
         _save(disk)
     return dict(choice)
 
