@@ -281,11 +281,19 @@ const void* eigh_kernel_for(int T, bool cta, unsigned* threads = nullptr) {
   return (const void*)lrd::eigh_reg_kernel<64>;
 }
 
-// Whether small launches of this frame count have a kernel of their own.
-// Eigensolve phase on B200 at T = 48, without / with it: one matrix 0.105 / 0.085 ms, 1176
-// matrices 0.109 / 0.087. It runs where the launch fits the device at its eight warps
-// per SM; above, twelve warps hide each other's latency (12600 matrices 0.73).
-bool eigh_wide(int T, bool cta) { return !cta && T > 32 && T <= 48; }
+// The kernel for small launches of this frame count (nullptr: none). It runs where the
+// launch fits the device at its eight warps per SM. Eigensolve phase on B200, ms without
+// / with it: T = 48, one matrix 0.106 / 0.086, 600 0.109 / 0.088, 1560 0.124 / 0.103, 2304
+// 0.127 / 0.104 (T = 36 and 40 likewise), and 2464, where it would not fit, 0.143 / 0.178;
+// T = 32, one 0.070 / 0.065, 300 0.082 / 0.077, 4400 0.095 / 0.092, and 5760 0.114 / 0.153.
+// Up to T = 32 only where the solve has the device to itself: beside the other kernels
+// of the host pipeline its registers cost more than they gain (96x96x48x32 / 5^3 /
+// stride 2 from pinned memory 2.22 / 2.31 ms); at T = 48 they gain there too (headline 3.01
+// / 2.95 ms).
+const void* eigh_wide_for(int T, bool cta) {
+  if (cta || T > 48) return nullptr;
+  return T <= 32 ? (const void*)lrd::eigh_reg_wide_kernel<32> : (const void*)lrd::eigh_reg_wide_kernel<48>;
+}
 
 template <int TPT, int SPLIT>
 void* recon_fn(bool accurate) {
@@ -532,8 +540,9 @@ int run_eigh(const lrd_plan* P, char* ws, const float* d_gram, float* d_vecs, fl
     void* eargs[] = {(void*)&gin, (void*)&vout, (void*)&lout, (void*)&r,      (void*)&w,   (void*)&s2,
                      (void*)&tv,  (void*)&nvv,  (void*)&p0v,  (void*)&rcount, (void*)&rids, (void*)&nmat};  // nmat: the warp kernels
     const long long blocks = (nb + mats - 1) / mats;
-    if (eigh_wide(T, P->eigh_cta) && blocks <= (long long)lrd::kEighWideBlocks * P->sms)
-      efn = (const void*)lrd::eigh_reg_wide_kernel<48>;
+    const void* wide = eigh_wide_for(T, P->eigh_cta);
+    const bool alone = queue < 0;  // (the pipelines' slabs have queues of their own)
+    if (wide != nullptr && (alone || T > 32) && blocks <= (long long)lrd::kEighWideBlocks * P->sms) efn = wide;
     cudaError_t le = cudaLaunchKernel(efn, dim3((unsigned)blocks), dim3(eth), eargs, P->smem_eigh, st);
     if (le != cudaSuccess) return cuda_fail(le, "eigh kernel launch");
     int rc = launch_check("eigh kernel launch");
@@ -860,7 +869,7 @@ int create_plan(const lrd_problem* pr, const std::vector<int32_t>* x_corners, lr
     }
   }
   if (!rc) rc = set_smem(eigh_kernel_for(T, P->eigh_cta), P->smem_eigh);
-  if (!rc && eigh_wide(T, P->eigh_cta)) rc = set_smem((const void*)lrd::eigh_reg_wide_kernel<48>, P->smem_eigh);
+  if (const void* wide = eigh_wide_for(T, P->eigh_cta); !rc && wide != nullptr) rc = set_smem(wide, P->smem_eigh);
   if (!rc && P->recon_warp) rc = set_smem(recon_warp_ptr(T, pr->form != LRD_FORM_PLAIN), lrd::recon_warp_smem_bytes(T));
   if (!rc && !P->recon_tc) rc = set_smem(recon_kernel_ptr(P->tpt, P->split, false), P->smem_recon);
   if (!rc && !P->recon_tc) rc = set_smem(recon_kernel_ptr(P->tpt, P->split, true), P->smem_recon);
