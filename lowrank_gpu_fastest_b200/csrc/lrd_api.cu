@@ -637,7 +637,7 @@ int validate_problem(const lrd_problem* pr) {
 // brick when set (a brick must fit the reconstruction kernel's threads per
 // CTA). Without either, frame counts the warp kernel is built for take it
 // (``warp``; recon_warp_brick()).
-// Measured on B200, reconstruction ms, 96x96x48x48 / 11^3 / stride 3:
+// Measured on B200, reconstruction phase ms, 96x96x48x48 / 11^3 / stride 3:
 // brick kernel (3x3x3, 2 threads per voxel) 1.22 -> warp kernel 0.83.
 int pick_layout(const lrd_problem* pr, const int dims[3], const int pat[3], const std::vector<int32_t> corners[3],
                 int& rsplit, int& rtpt, int best[3], bool* warp = nullptr, bool* tc = nullptr) {

@@ -26,8 +26,8 @@
 //    in chunks: consecutive patches along z whose rows of v_k fit a shared-memory
 //    buffer, brought there by one bulk copy per patch (the p x T block is
 //    contiguous) while the chunk before is used; one barrier per chunk (four warps
-//    a CTA waited 17% of the time at it: headline 0.86 ms against 0.80; one warp
-//    0.85). Ranks and weights of a chunk are loaded one per lane, a chunk ahead.
+//    a CTA waited 17% of the time at it, 7% slower at the headline; one warp
+//    6%). Ranks and weights of a chunk are loaded one per lane, a chunk ahead.
 //    Read straight from global memory, a row costs a warp four clocks of the SM's
 //    data path per 16 bytes a lane, whatever the lanes share, and an L1 or L2
 //    latency per patch (half of all stall cycles); neighbouring lanes here belong
@@ -38,11 +38,11 @@
 // The float64 sums of ACCURATE take one voxel per lane (LPV = 4): 16 frames of two
 // voxels would need 64 registers for the sums alone.
 //
-// Reconstruction on B200, one voxel per lane from global memory -> here: headline
-// 1.085 -> 0.80 ms (accurate 1.365 -> 1.03), dense 5^3 at T = 32 1.92 -> 1.52, 7^3 at T =
-// 64 2.14 -> 1.28, T = 96 1.11 -> 0.74, 128x128x64x96 / 11^3 / stride 2 17.0 -> 11.1. Per
+// Reconstruction phase on B200, one voxel per lane from global memory -> here: headline
+// 1.10 -> 0.83 ms (accurate 1.365 -> 1.08), dense 5^3 at T = 32 1.92 -> 1.65, 7^3 at T =
+// 64 2.14 -> 1.31, T = 96 1.11 -> 0.76, 128x128x64x96 / 11^3 / stride 2 17.0 -> 11.5. Per
 // patch of rank 4 a warp issues about 220 instructions for two 16-voxel
-// contractions of 96 packed FMAs; the FMA pipe is 40% busy, issue 50%.
+// contractions of 96 packed FMAs; the FMA pipe is 44% busy, issue 52%.
 //
 // The brick a CTA covers is recon_warp_brick()'s in the plan's brick grid, so the
 // host pipeline and slab sharding address it exactly like recon_kernel's bricks.
@@ -445,13 +445,17 @@ __device__ __forceinline__ void recon_warp_body(const float* __restrict__ xc, co
   }
 }
 
-// CTAs per SM, which cap the registers. Measured on B200, reconstruction ms with 6 /
-// 8 / 10: 96x96x48x32 / 5^3 / stride 1 1.83 / 1.60 / 1.52; 96x96x48x48 / 11^3 / stride 3
-// 0.827 / 0.800 / 1.28 (accurate 1.24 / 1.08 / 1.03); 101x87x43x64 / 7^3 / stride 2 1.28
-// / 2.66 / 3.08 (spills); 64x64x48x96 / 11^3 / stride 3 0.74 / 0.84 / 1.33.
+// CTAs per SM, which cap the registers. Reconstruction phase on B200, ms with 6 / 8 /
+// 10, at 96x96x48xT / 11^3 / stride 3 and 64x64x32xT / 5^3 / stride 1:
+//   T = 32  plain 0.735 / 0.651 / 0.670, 0.781 / 0.705 / 0.733 (372416 patches of 5^3 1.94 / 1.68 / 1.65)
+//           accurate 0.904 / 0.930 / 0.858, 0.840 / 0.865 / 0.815
+//   T = 48  plain 0.867 / 0.835 / 1.30, 0.924 / 0.890 / 1.32; accurate 1.23 / 1.08 / 1.14, 1.14 / 1.02 / 1.03
+//   T = 64  plain 1.07 / 2.57 / 3.05 (spills), 1.11 / 2.49 / 3.08; accurate 1.45 / 1.47 / 3.58, 1.35 / 1.37 / 3.05
+//   T = 96  plain 1.65 / 1.92 / 3.64, 1.47 / 1.65 / 3.13; accurate 1.85 / 3.67 / 4.24, 1.73 / 3.34 / 3.96
+// and at 80x70x40xT / 7^3 / 2 and 64x64x40xT / 11^3 / 2 alike.
 template <int T, bool ACCURATE>
 __host__ __device__ constexpr int recon_warp_ctas() {
-  return T == 32 || (T == 48 && ACCURATE) ? 10 : T == 48 || (T == 64 && ACCURATE) ? 8 : 6;
+  return T == 32 ? 10 : T == 48 ? 8 : 6;
 }
 
 template <int T, bool ACCURATE>
