@@ -134,7 +134,8 @@ def reference_step0():
 
 def phase_kernel(phase, T, form):
     """Kernel that a plan phase launches for T frames (the eigensolve phase
-    also runs the refine kernel and its cursor, both under 0.5% of it)."""
+    also runs the near-tie pass: under 0.5% of it with an empty queue, one
+    patch's latency with one queued)."""
     if phase == "gram":
         return "gram_tc_kernel" if (form in ("tensor", "tensor_bf16") and T <= 64) else "gram_z_kernel"
     if phase == "eigh_mp":
@@ -142,7 +143,7 @@ def phase_kernel(phase, T, form):
     if phase == "recon" and form in ("tensor", "tensor_bf16") and T % 4 == 0 and 8 <= T <= 64:
         return "recon_tc_kernel"  # tcgen05, 4x4x8 voxel bricks
     if phase == "recon" and T in (32, 48, 64, 96):
-        return "recon_warp_kernel"  # one warp per 2x2x2 voxel block (the plan's default layout)
+        return "recon_warp_kernel"  # two warps per brick of 2x2x8 or 2x2x4 voxels (the plan's default layout)
     if phase == "recon" and form == "plain" and 45 <= T <= 48:
         return "recon_kernel_t24s2"  # 24 frames x 2 threads, built with 112 registers
     return {"center": "center_kernel", "recon": "recon_kernel"}[phase]
@@ -791,8 +792,9 @@ def executed_fp32(ph, shape, patch, stride, ranks, fp32_peak, form):
     """FP32 work the Gram and reconstruction kernels execute (not the 2 N T^2
     per patch of the full-square algorithmic count), over their phase times,
     as a fraction of the measured SGEMM rate: the column Gram forms each
-    z-plane's Gram once per (x, y) column on the upper triangle in 4x4 blocks
-    and adds it into the windows; the reconstruction does y = (x - m) V_p^T
+    z-plane's Gram once per (x, y) column on the upper triangle, counted here in
+    4x4 blocks (its 8x8 blocks execute 8% more at T = 48), and adds it into the
+    windows; the reconstruction does y = (x - m) V_p^T
     and y V_p (4 p T flops) for every covered voxel-patch pair."""
     from lowrank_gpu_fastest_b200.problem import axis_corners
 

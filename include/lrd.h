@@ -246,7 +246,7 @@ int lrd_denoise_static(const lrd_problem* problem, const float* d_vol, float* d_
  * with the same pointers replay it as a single graph launch (different
  * pointers re-capture). No host synchronisation on the replay path. One call
  * at a time per batch plan. lrd_batch_num_launches gives the kernel launches
- * of one call (18 for the 24 mixed-shape volumes of the batched benchmark,
+ * of one call (16 for the 24 mixed-shape volumes of the batched benchmark,
  * against 5 per volume one by one). */
 typedef struct lrd_batch_plan lrd_batch_plan;
 int lrd_batch_plan_create(const lrd_problem* problems, int32_t n, int32_t n_streams, lrd_batch_plan** plan);

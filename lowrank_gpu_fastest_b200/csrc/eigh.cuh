@@ -2,13 +2,12 @@
 //
 // Replaces the ladder's ``torch.linalg.eigh`` (step8_tuned.py:134; cuSOLVER),
 // ``mp_keep`` (step8_tuned.py:96-113), the projector bmm (step8:136) and the
-// weight (step8:137). One warp owns one patch's Gram matrix in shared memory:
+// weight (step8:137). For each patch's Gram matrix:
 //
 //  1. exact power-of-two scaling so the largest diagonal entry is in [0.5, 1);
-//  2. Householder reduction to tridiagonal form (lower, one reflector per
-//     column; the reflector vectors stay in the strictly-lower part);
-//  3. every eigenvalue by bisection on Sturm counts, two eigenvalues per lane
-//     evaluated as two interleaved dependency chains;
+//  2. Householder reduction to tridiagonal form, one reflector per column;
+//  3. every eigenvalue from Sturm counts, its interval cut at one or several
+//     points a round;
 //  4. the MP rank from the full spectrum, evaluated like step0_numpy_loop.py:
 //     18-24: eigs = float32(max(lambda, 0) / N) in descending order with the
 //     smallest (null) eigenvalue dropped (step4_gram_eigh.py:49), float32
@@ -16,21 +15,23 @@
 //       float64(float32(eigs_i - eigs_last)) * (t - i) * (N - i)
 //         > float64(float32(4 * rcum_i)) * sqrt(float64(t * N))
 //     counted over all i (NumPy promotes the ladder's test to float64);
-//  5. the top-p eigenvectors, in chunks of 8: inverse iteration on the
-//     tridiagonal matrix (partial-pivoting LU, three solves from distinct
-//     pseudo-random starts), the Householder back-transform, then modified
-//     Gram-Schmidt in descending eigenvalue order;
+//  5. the top-p eigenvectors, a few at a time: those of the tridiagonal matrix,
+//     the Householder back-transform, then modified Gram-Schmidt in descending
+//     eigenvalue order;
 //  6. w = float32(1 / (2 + p)) (step0:36).
 //
-// The main pass runs these steps in float32 on the float32 Gram
-// (eigh_reg.cuh, eigh_cta.cuh). A patch whose MP test has an index with
-// |lhs/rhs - 1| below kRefineTol (a near-tie that float32 round-off could
-// decide either way) is queued, and eigh_refine_kernel redoes it in float64:
-// each voxel's time course centred in float64 from the input volume (the
+// The main pass runs these steps in float32 on the float32 Gram, the matrix in the
+// registers of a warp's lanes or of a CTA's threads, its vectors by twisted
+// factorisations (eigh_reg.cuh, eigh_cta.cuh). A patch whose MP test has an index
+// with |lhs/rhs - 1| below kRefineTol (a near-tie that float32 round-off could
+// decide either way), or one of whose kept vectors float32 could not tell from an
+// earlier one, is queued, and eigh_refine_kernel (eigh_refine.cuh) redoes it in
+// float64: each voxel's time course centred in float64 from the input volume (the
 // float64 mean of its float32 values), the Gram from float64 products with a
-// float64 sum, then the same eigen/MP/eigenvector steps in float64 - so
-// near-ties are decided as the float64 evaluation of the algorithm decides
-// them, down to margins far below the float32 centred data's own rounding.
+// float64 sum, then the same steps in float64, the vectors by inverse iteration
+// (partial-pivoting LU) from pseudo-random starts - so near-ties are decided as
+// the float64 evaluation of the algorithm decides them, down to margins far
+// below the float32 centred data's own rounding.
 //
 // Output per patch: the p eigenvectors (descending eigenvalue order) as the
 // rows of a compact p x T block at the start of the patch's T x T slot (the
@@ -51,7 +52,6 @@ struct Num<float> {
   static __device__ __forceinline__ float eps() { return FLT_EPSILON * 0.5f; }
   static __device__ __forceinline__ float tiny() { return FLT_MIN; }
   static __device__ __forceinline__ float huge() { return FLT_MAX; }
-  static __device__ __forceinline__ float fdiv(float a, float b) { return __fdividef(a, b); }
   static __device__ __forceinline__ float rsq(float a) { return rsqrtf(a); }
 };
 template <>
@@ -59,7 +59,6 @@ struct Num<double> {
   static __device__ __forceinline__ double eps() { return DBL_EPSILON * 0.5; }
   static __device__ __forceinline__ double tiny() { return DBL_MIN; }
   static __device__ __forceinline__ double huge() { return DBL_MAX; }
-  static __device__ __forceinline__ double fdiv(double a, double b) { return a / b; }
   static __device__ __forceinline__ double rsq(double a) { return rsqrt(a); }
 };
 
@@ -93,8 +92,8 @@ __device__ __forceinline__ float start_entry(int i, int j) {
   return (float)(h >> 8) * (2.0f / 16777216.0f) - 1.0f;
 }
 
-constexpr int kInvGroup = 8;  // eigenvectors refined concurrently (one lane each)
-constexpr int kInvSolves = 2;  // float32 solvers: inverse-iteration solves per eigenvector
+constexpr int kInvGroup = 8;  // eigenvectors formed at once, at most
+constexpr int kInvSolves = 2;  // float64 pass: inverse-iteration solves per eigenvector
 
 // Floats of the packed Householder reflector rows of the float32 solvers: row
 // k (k < n - 2 <= TMAX - 2) is stored from its first live 4-column group on,

@@ -875,7 +875,9 @@ __device__ __forceinline__ void eigh_reg_body(const float* gram, float* vecs, fl
   LRD_STAMP(7);
 }
 
-// Warps per SM by the registers the rows need (R TMAX and about 50 more).
+// Warps per SM: 168 registers, what 32 x 4, 48 x 3 and 64 x 2 row entries and the
+// rest leave with few spills (bytes stored / loaded, alone and in the packed launch:
+// T = 32 20 / 44 and 24 / 24, T = 48 208 / 240 and 324 / 244, T = 64 88 / 52 and 8 / 8).
 template <int TMAX>
 __host__ __device__ constexpr int eigh_reg_min_blocks() {
   return 12;

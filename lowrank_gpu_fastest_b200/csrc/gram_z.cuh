@@ -22,8 +22,8 @@
 // SM that stop at the plane barrier and at the flush below. Gram phase on B200:
 // 96x96x48x48 / 11^3 / stride 3 0.61 -> 0.52 ms, 96x96x48x32 / 5^3 / stride 1 1.58
 // -> 1.40, 101x87x43x64 / 7^3 / stride 2 1.21 -> 0.98, 64x64x48x96 / 11^3 / stride 3
-// 0.99 -> 0.70; 128x128x64x96 / 11^3 / stride 2, whose full ring does not fit
-// shared memory and which ran a CTA per patch, 68.1 -> 10.2.
+// 0.99 -> 0.70; 128x128x64x96 / 11^3 / stride 2, whose ring of six windows (208 KB) passed
+// the kernel's former limit of 200 KB and which ran a CTA per patch, 68.1 -> 10.4.
 //
 // Planes that lie in the same windows (two of three at 11^3 / stride 3) are summed
 // in registers, at most gramz_group() of them; at the last the KS lanes' partial sums are

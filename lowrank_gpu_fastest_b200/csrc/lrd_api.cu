@@ -825,8 +825,13 @@ int create_plan(const lrd_problem* pr, const std::vector<int32_t>* x_corners, lr
     P->gramtc_ring = ring;
     P->gramz_ks = pr->gram_split > 0 ? 2 * pr->gram_split : gramz_split(T);
     while (P->gramz_ks > 2 && lrd::gramz_threads(T, P->gramz_ks) > lrd::kGramzMaxThreads) P->gramz_ks /= 2;
-    // The window ring, or the part of it that fits beside the planes (the
-    // columns are then cut into ranges of that many windows).
+    // The window ring, or the part of it that fits beside the planes (the columns are
+    // then cut into ranges of that many windows, whose shared planes are formed more
+    // than once). A cut column still beats a CTA per patch with the smallest ring.
+    // Gram ms, per patch / cut: 40x40x32x96 / 11^3 / stride 1 (ring 6 of 11) 14.0 / 2.6, T = 128
+    // 24.9 / 5.1; 64x64x48x119 / 11^3 / 2 (1 of 6) 21.5 / 8.5; 96x96x48x99 / 11^3 / 3 (2 of 5)
+    // 10.8 / 3.3; 64x64x48x96 / 15^3 / 3 (2 of 5) 6.5 / 2.1; 16x16x32x96 / 15^3 / 2, 40 patches (2
+    // of 8), 0.40 / 0.13; 40x40x32x64 / 15^3 / 1 (12 of 15) 13.7 / 1.9.
     P->gramz_ring = ring;
     while (P->gramz_ring > 1 && lrd::gramz_smem_bytes(pr->px, pr->py, T, P->gramz_ks, P->gramz_ring) > kSmemMax) --P->gramz_ring;
     P->gramz_cut = P->gramz_ring < ring ? (g.ncz + P->gramz_ring - 1) / P->gramz_ring : 1;

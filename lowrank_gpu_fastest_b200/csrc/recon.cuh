@@ -209,9 +209,12 @@ __device__ __forceinline__ void recon_body(const float* __restrict__ xc, const f
       const float4* vr = reinterpret_cast<const float4*>(vb + (size_t)kk * TP + t0);
       constexpr int CH = 4 / SPLIT;         // chunks per thread
       constexpr int CU4 = TPT / 4 / CH;     // float4 groups per chunk
-      // For the frame counts that have a warp kernel (chunks of 8, 12, 16 and 24
-      // frames) a chunk's even and odd frames are summed apart, as it does, and at T =
-      // 96 in two halves, which it gives to two lanes; other chunks in one sum.
+      // Chunks of 8, 12, 16 and 24 frames, those of the frame counts that have a warp
+      // kernel and of their neighbours (17..32, 33..48, 49..64, 81..96), have their even and odd
+      // frames summed apart, as it does, and at T = 96 in two halves, which it gives to
+      // two lanes; other chunks are one sum. The two sums cost nothing: reconstruction
+      // ms, one sum / two, 48x48x32 / 7^3 / stride 2 at T = 31 0.260 / 0.254, 47 0.403 / 0.389,
+      // 63 0.847 / 0.860, 91 1.895 / 1.897.
       constexpr bool EO = CU4 == 2 || CU4 == 3 || CU4 == 4 || CU4 == 6;
       float cp[CH];
       auto sum_even_odd = [&](int c, auto from, auto to) {  // frame quads [from, to) of chunk c
