@@ -20,8 +20,8 @@
 // FMA (two IEEE FMAs) halves the issue slots: 107 instead of 94 FMA a clock at 12
 // warps per SM in a loop of nothing else. What bounds it now is 9 to 12 warps per
 // SM that stop at the plane barrier and at the flush below. Gram phase on B200:
-// 96x96x48x48 / 11^3 / stride 3 0.61 -> 0.52 ms, 96x96x48x32 / 5^3 / stride 1 1.58
-// -> 1.40, 101x87x43x64 / 7^3 / stride 2 1.21 -> 0.98, 64x64x48x96 / 11^3 / stride 3
+// 96x96x48x48 / 11^3 / stride 3 0.61 -> 0.53 ms, 96x96x48x32 / 5^3 / stride 1 1.58
+// -> 1.43, 101x87x43x64 / 7^3 / stride 2 1.21 -> 1.00, 64x64x48x96 / 11^3 / stride 3
 // 0.99 -> 0.70; 128x128x64x96 / 11^3 / stride 2, whose ring of six windows (208 KB) passed
 // the kernel's former limit of 200 KB and which ran a CTA per patch, 68.1 -> 10.4.
 //

@@ -144,14 +144,15 @@ constexpr long long kIoSlabBytes = 7ll << 19;
 namespace {
 
 // Voxel-row split of the column Gram (threads per 8 x 8 block). Measured on
-// B200, Gram phase ms with 2 / 4 / 8: 96x96x48x48, 11^3, stride 3 0.80 / 0.52 /
-// 0.52 (48x48x24x48 0.125 / 0.097 / 0.090: 8 there); 96x96x48x32, 5^3, stride 1
-// 1.77 / 1.40 / 1.69; 101x87x43x64, 7^3, stride 2 1.17 / 0.98 / 1.50;
-// 64x64x48x96, 11^3, stride 3 0.90 / 0.70 / -. A CTA of fewer than 48 threads at
-// 4 (T <= 24) takes 8. Frame counts not a multiple of 4 take 4: 48x48x40 / 7^3 / stride
-// 2 at T = 17, 31, 53, 65, 127 0.15 / 0.09 / 0.10, 0.23 / 0.15 / 0.15, 0.45 / 0.29 /
-// 0.31, 0.73 / 0.48 / 0.50, 1.94 / 1.40 / -. The split does not depend on the launch: it changes the
-// rounding.
+// B200, Gram phase ms with 2 / 4 / 8: 96x96x48x48, 11^3, stride 3 0.70 / 0.54 /
+// 0.53 (48x48x24x48 0.128 / 0.098 / 0.089, 64x64x40x40 0.209 / 0.166 / 0.139: 8 around there,
+// though 64x64x40x56, 7^3, stride 2 has 0.41 / 0.34 / 0.38); 96x96x48x32, 5^3, stride 1 1.41
+// / 1.44 / 1.69; 101x87x43x64, 7^3, stride 2 1.16 / 1.00 / 1.48; 64x64x48x96, 11^3, stride 3
+// 0.94 / 0.70 / -. A CTA of fewer than 48 threads at 4 (T <= 24) takes 8: 64x64x32x16, 5^3, stride
+// 2 0.096 / 0.068 / 0.051, but x24, 7^3 0.145 / 0.092 / 0.104. Frame counts not a multiple of 4
+// take 4: 48x48x40 / 7^3 / stride 2 at T = 17, 31, 53, 65, 127 0.13 / 0.08 / 0.09, 0.17 / 0.14 / 0.13,
+// 0.35 / 0.28 / 0.29, 0.57 / 0.46 / 0.47, 1.79 / 1.36 / -. The split does not depend on the launch:
+// it changes the rounding.
 int gramz_split(int T) { return !lrd::gramz_exact(T) && (T <= 24 || (T > 40 && T <= 56)) ? 8 : 4; }
 
 void* gramtc_kernel_ptr(bool bf16) {
